@@ -143,13 +143,13 @@ void mc_b200_clear_error(void);
 uint32_t mc_b200_last_bad_blocks(void);
 /* How the calling thread's decodes without a plan (per-call chunk, block and
  * region reads, the host-blob pipeline) split the entropy stage between its
- * two kernels. A lane of a warp decodes a block at about 5 issue slots per
- * bin but about 450 cycles per bin; one thread alone takes about 25 slots but
- * about 120 cycles. share > 1: the longest coded/share blocks on single
- * threads, the rest one per lane; 1: every block on a single thread; 0: every
- * block on a lane; -1 (the default): by the launch's coded-block count (every
- * block on single threads up to 28 K blocks, the longest 1/64 up to 90 K), and
- * lanes only in the host-blob pipeline, whose groups overlap. Decoded voxels
+ * two kernels. A lane of a warp decodes a block at a fraction of the issue
+ * slots, one thread alone in less time. share > 1: the longest coded/share
+ * blocks on single threads, the rest one per lane; 1: every block on a single
+ * thread; 0: every block on a lane; -1 (the default): by the launch's
+ * coded-block count (every block on single threads up to 15 K blocks, the
+ * longest four per SM up to 200 K), and lanes only in the host-blob pipeline,
+ * whose groups overlap. Decoded voxels
  * are the same in every case. Returns 0; -1 (with the last error set) for
  * share < -1 or without a usable device. No reference counterpart. */
 int  mc_b200_set_entropy_solo(int share);

@@ -208,10 +208,10 @@ LaunchCfg autotune(DecodeBatch &B, float q, int nblocks, cudaStream_t s) {
     pick(8, [](LaunchCfg &c, int i) { c.ent_warps = ent_shape[i][0]; c.ent_ctas_per_sm = ent_shape[i][1]; }, 0);
     static const int ent_claim[] = {1, 2, 4};
     pick(3, [](LaunchCfg &c, int i) { c.ent_claim = ent_claim[i]; }, 0);
-    // the longest 1/64 .. 1/8 of the blocks on single-thread warps, none, or
+    // the longest 1/384 .. 1/16 of the blocks on single-thread warps, none, or
     // all of them (the single-thread kernel)
-    static const int ent_solo[] = {0, 64, 32, 16, 8, 1};
-    pick(6, [](LaunchCfg &c, int i) { c.ent_solo = ent_solo[i]; }, 0);
+    static const int ent_solo[] = {0, 384, 128, 64, 32, 16, 1};
+    pick(7, [](LaunchCfg &c, int i) { c.ent_solo = ent_solo[i]; }, 0);
     static const int rec_opts[] = {3, 4, 5};
     pick(3, [](LaunchCfg &c, int i) { c.rec_ctas_per_sm = rec_opts[i]; }, 1);
     // the whole decode: separate kernels, the long blocks on a second

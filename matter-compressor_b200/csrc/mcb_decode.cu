@@ -3,11 +3,12 @@
 // Stage 1, k_entropy: one LANE per block. The adaptive binary range decoder
 // is a serial dependency chain per block (src/mc_codec.c:197-226), so the
 // parallelism is across blocks: every lane of a warp runs its own decoder and
-// the loop body decodes exactly one bin per lane per iteration (a flat state
-// machine), so lanes never wait on each other inside a block. The per-bin
-// chain is kept short: the significance band is tracked by scan-position
-// boundaries and the density by a running count, so the only shared-memory
-// read on the chain is the context itself. The lane's adaptive contexts sit
+// the loop body advances every lane by up to a whole coefficient -- a run of
+// zeros, a significance bin, a magnitude rung and a sign -- in straight-line
+// code, so lanes never wait on each other inside a block. The per-bin chain is
+// kept short: the significance band is tracked by scan-position boundaries and
+// the density by the positions at which the last three ones leave its window,
+// so the only shared-memory read on the chain is the context itself. The lane's adaptive contexts sit
 // in shared memory as 32-bit words (context j of lane l at word j*32+l:
 // conflict-free). Output per block: a small header (dc, flags) and a list of
 // nonzero levels plus corrections.
@@ -38,45 +39,42 @@ __constant__ float c_cos[16][16];
 __constant__ uint16_t c_bend[9];
 
 // ---------------------------------------------------------------- stage 1
-// Lane states. The three fast states cover every bin of the coefficient loop
-// and share one branch-free step that every lane of a warp runs together; the
-// slow states occur a few times per block and are worked off by the lanes
-// that hold them while the rest of the warp waits (see run_lanes). S_IDLE is
-// a parked lane, a fixed point of the fast step (see park). The block header
-// and EOB are decoded when a lane starts its block.
+// Lane states. A lane that decodes significance and magnitude bins takes part
+// in the step that every lane of a warp runs together; the slow states occur a
+// few times per block and are worked off by the lanes that hold them while the
+// rest of the warp waits (see run_lanes). The block header and EOB are decoded
+// when a lane starts its block.
 enum : uint32_t {
-    F_SIG = 0,   // significance of scan position p: context sigb + min(popcount(last 16 flags), 3)
-    F_MAG,       // unary magnitude rung k: context 56 + k
-    F_BYP,       // a bypass bin: the sign of the coefficient at p (m != 0), an Exp-Golomb prefix
-                 // bit (m == 0, rem == 0; k counts 12 + the one-bits) or a suffix bit (rem != 0)
+    F_RUN = 0,   // k == 0: significance of scan position p, context sigb + min(ones among the last 16
+                 // flags, 3); k in 1..11: magnitude rung k of the coefficient at p - 1, context 56 + k;
+                 // k >= 12: a bit of the Exp-Golomb prefix behind the twelfth rung, 12 + the ones so far
     S_IDLE,      // no more blocks for this lane
+    S_LAST,      // the coefficient at the last position before the EOB, significant by definition
     S_END,       // scan done: corrections, then the block is finished
-    S_EGS,       // an Exp-Golomb suffix of more than 16 bits (only corrupt streams)
     S_DONE
 };
-// Context slots per lane: the 68 adaptive contexts plus one scratch slot that
-// bypass bins read and write in place of a real context. The scratch slot
-// directly follows the magnitude ladder, so "the next rung" of rung 11 is it.
+// Context slots per lane: the 68 adaptive contexts plus one that follows the
+// magnitude ladder and holds 1: a bypass bin splits at (range >> 1) * 1 where a
+// rung splits at (range >> 12) * p. A parked lane uses it as a scratch slot.
 constexpr int kCtxSlots = kNumCtx + 1;
 constexpr uint32_t kScr = kNumCtx;
 static_assert(kScr == kCtxMag + 12, "scratch slot follows the 12 magnitude rungs");
-// Exp-Golomb prefixes count in k from this base (the magnitude ladder hands
-// over at its 12th rung with k = 12).
-constexpr uint32_t kEgBase = 12;
-// Byte-permute selector that shifts code left one byte and brings in byte i
-// of the window: result = {code.b2, code.b1, code.b0, w.b[i]}; i = sel - kSel0.
-constexpr uint32_t kSel0 = 0x2104u;
+// The range is renormalised when it falls below this (src/mc_codec.c:202).
+constexpr uint32_t kTop = 1u << 24;
 
 struct LaneState {
     const uint8_t *abase;      // payload start rounded down to 4 bytes
     uint32_t *ent;             // the block's entries in the arena (first cap of them)
     uint32_t len, off0;        // payload length, payload start - abase
-    uint32_t w, nxt, sel, jn;  // window word, next word (raw), byte selector, index of the next word
-    uint32_t nmask;            // the next word's payload bytes (applied when it enters the window)
+    uint32_t w, w2, used;      // two payload words, first byte highest; bits of w already read (0, 8, 16, 24)
+    uint32_t nxt, nmask, jn;   // the word after them (raw), its payload bytes, its index
     uint32_t code, range;
-    uint32_t st, p, eob, hist, sigb, band, bend, stop;   // hist: significance flags, newest in bit 0
-    uint32_t k, m, rem, acc;   // rung / prefix count, magnitude of the pending sign, suffix bits left and read
-    uint32_t cc, pc;           // context slot of the next bin and its probability
+    uint32_t st, p, eob, sigb, band, bend, stop;   // p: next scan position to decode a significance flag of
+    uint32_t e1, e2, e3;       // the last three significant positions (newest first) + 17: the position
+                               // from which each has left the 16-flag density window
+    uint32_t cs, ps, lim;      // significance context slot at p, its probability, and the position from
+                               // which another slot (or a position event) is due
+    uint32_t k, pm;            // next magnitude rung (0 at a significance bin), its probability
     uint32_t hdr;              // flag0, flag1, dc bits 7..0 (10 bits, first bin highest)
     uint32_t nent, cap, ovf, bad, ccount;
     int item;
@@ -98,28 +96,30 @@ __device__ __forceinline__ uint32_t word_raw(const LaneState &L, uint32_t j) {
     return v;
 }
 __device__ __forceinline__ uint32_t load_word(const LaneState &L, uint32_t j) {
-    return word_raw(L, j) & word_mask(L, j);
+    return __byte_perm(word_raw(L, j) & word_mask(L, j), 0, 0x0123);
 }
 
+// The window's first word is read to its end: the second takes its place.
 __device__ __forceinline__ void refill(LaneState &L) {
-    L.w = L.nxt & L.nmask;
-    L.sel = kSel0;
+    L.w = L.w2;
+    L.w2 = __byte_perm(L.nxt & L.nmask, 0, 0x0123);
+    L.used -= 32;
     ++L.jn;
     L.nmask = word_mask(L, L.jn);
     L.nxt = word_raw(L, L.jn);
 }
 
-// One payload byte (slow paths). The window always holds an unread byte:
-// consuming the last one refills it at once.
+// One payload byte (slow paths).
 __device__ __forceinline__ uint32_t next_byte(LaneState &L) {
-    const uint32_t b = (L.w >> (8 * (L.sel - kSel0))) & 0xFFu;
-    if (++L.sel == kSel0 + 4) refill(L);
+    const uint32_t b = (L.w >> (24 - L.used)) & 0xFFu;
+    L.used += 8;
+    if (L.used == 32) refill(L);
     return b;
 }
 
 // Renormalise (src/mc_codec.c:202).
 __device__ __forceinline__ void renorm(LaneState &L) {
-    while (L.range < (1u << 24)) { L.code = (L.code << 8) | next_byte(L); L.range <<= 8; }
+    while (L.range < kTop) { L.code = (L.code << 8) | next_byte(L); L.range <<= 8; }
 }
 
 // One adaptive bin (src/mc_codec.c:198-204).
@@ -188,34 +188,36 @@ __device__ __forceinline__ bool put_entry(LaneState &L, const EntParams &P, uint
     return true;
 }
 
-// Context slot of the bin the lane's state asks for next and its current
-// value; bypass bins use the scratch slot.
-__device__ __forceinline__ void load_ctx(LaneState &L, const uint32_t *ctx) {
-    L.cc = L.st == F_SIG ? L.sigb + min((uint32_t)__popc(L.hist & 0xFFFFu), 3u)
-                         : (L.st == F_MAG ? (uint32_t)kCtxMag + L.k : kScr);
-    L.pc = ctx[L.cc * 32];
+// The density class at position p, min(ones among the last 16 flags, 3)
+// (src/mc_codec.c:249-259), from the expiries of the last three ones: its
+// context slot, and the position up to which slot and band stay the same.
+__device__ __forceinline__ void density(LaneState &L) {
+    const bool a3 = L.p < L.e3, a2 = L.p < L.e2, a1 = L.p < L.e1;   // e1 >= e2 >= e3
+    L.cs = L.sigb + (a3 ? 3u : (a2 ? 2u : (a1 ? 1u : 0u)));
+    L.lim = min(L.stop, a3 ? L.e3 : (a2 ? L.e2 : (a1 ? L.e1 : 0xFFFFFFFFu)));
 }
 
 // flags bit 1 (has corrections) is the second header bin
 __device__ __forceinline__ bool has_corr(const LaneState &L) { return (L.hdr >> 8) & 1; }
 
-// A lane with no more work: a fixed point of fast_step. With code 0, range
-// 0xFFFFF000 and probability 4096 on the scratch slot, every step decodes a
-// 0 that leaves range, probability and selector as they are, so the lane
-// reads nothing, stores nothing and raises no event.
+// A lane with no more work: an endless run of zeros over an empty payload, in
+// the scratch context (code 0 is below every split; p stays far from stop).
 __device__ __forceinline__ void park(LaneState &L) {
     L.st = S_IDLE;
     L.item = -1;
     L.code = 0;
-    L.range = 0xFFFFF000u;
-    L.pc = 4096;
-    L.cc = kScr;
-    L.sel = kSel0;
-    L.m = 0;
-    L.rem = 0;
+    L.range = 0xFFFFFFFFu;
+    L.sigb = L.cs = kScr;
+    L.ps = L.pm = 2048;
+    L.p = 0;
+    L.lim = L.stop = 0xFFFFFFFFu;
+    L.e1 = L.e2 = L.e3 = 0;
+    L.len = L.off0 = L.jn = 0;
+    L.w = L.w2 = L.nxt = L.nmask = L.used = 0;
+    L.k = 0;
 }
 
-// Scan position L.p is current and L.p >= L.stop: a band change and/or the
+// Scan position L.p is next and L.p >= L.stop: a band change and/or the
 // end of the scan. The last position before the EOB is significant by
 // definition and costs no bin (src/mc_codec.c:364); past the EOB the
 // coefficient loop ends.
@@ -223,15 +225,15 @@ __device__ __forceinline__ void position_event(LaneState &L, const uint32_t *ctx
     while (L.p >= L.bend) { L.band++; L.sigb += 4; L.bend = s_bend[L.band]; }
     if (L.p + 1 >= L.eob) {
         if (L.p + 1 == L.eob) {
-            L.hist = (L.hist << 1) | 1u;
-            L.st = F_MAG;
-            L.k = 0;
+            L.p++;
+            L.st = S_LAST;
         } else {
             L.st = S_END;
         }
     }
     L.stop = min(L.bend, L.eob - 1);   // eob >= 1 here (eob == 0 never enters the scan)
-    load_ctx(L, ctx);
+    density(L);
+    L.ps = ctx[L.cs * 32];
 }
 
 // Starts block `slot`: contexts from the quality table, range decoder,
@@ -244,6 +246,7 @@ __device__ __forceinline__ void lane_begin(LaneState &L, const EntParams &P, uin
     L.abase = reinterpret_cast<const uint8_t *>(src & ~(uintptr_t)3);
     L.off0 = (uint32_t)(src & 3);
     L.len = it.len;
+    ctx[kScr * 32] = 1;
     L.ent = P.arena + P.base[slot];
     L.cap = entry_cap(L.len);
     L.ovf = 0xFFFFFFFFu;
@@ -251,7 +254,8 @@ __device__ __forceinline__ void lane_begin(LaneState &L, const EntParams &P, uin
     L.nent = 0;
     L.ccount = 0;
     L.hdr = 0;
-    L.p = 0; L.eob = 0; L.hist = 0; L.k = 0; L.m = 0; L.rem = 0; L.acc = 0;
+    L.p = 0; L.eob = 0; L.k = 0;
+    L.e1 = 0; L.e2 = 0; L.e3 = 0;
     L.band = 0; L.sigb = kCtxSig; L.bend = s_bend[0]; L.stop = 0;
     if (L.len == 0) { L.st = S_DONE; return; }   // absent block: zeros
     const uint4 *q = reinterpret_cast<const uint4 *>(P.qtab[it.qslot].ctx);
@@ -267,10 +271,11 @@ __device__ __forceinline__ void lane_begin(LaneState &L, const EntParams &P, uin
         }
     }
     L.w = load_word(L, 0);
-    L.sel = kSel0 + L.off0;
-    L.jn = 1;
-    L.nmask = word_mask(L, 1);
-    L.nxt = word_raw(L, 1);
+    L.w2 = load_word(L, 1);
+    L.used = 8 * L.off0;
+    L.jn = 2;
+    L.nmask = word_mask(L, 2);
+    L.nxt = word_raw(L, 2);
     L.range = 0xFFFFFFFFu;
     L.code = 0;
     for (int i = 0; i < 5; ++i) L.code = (L.code << 8) | next_byte(L);
@@ -280,7 +285,8 @@ __device__ __forceinline__ void lane_begin(LaneState &L, const EntParams &P, uin
     const uint32_t eob = k < 2 ? k : (1u << (k - 1)) | bypass_bits(L, k - 1);
     L.eob = eob > (uint32_t)kN3 ? (uint32_t)kN3 : eob;
     if (L.eob == 0) { L.st = S_END; return; }
-    L.st = F_SIG;
+    L.st = F_RUN;
+    L.pm = ctx[kCtxMag * 32];
     position_event(L, ctx, s_bend);
 }
 
@@ -319,31 +325,49 @@ __device__ __forceinline__ void decode_corrections(LaneState &L, const EntParams
     }
 }
 
-// The slow states of one lane, run while the rest of its warp waits.
-__device__ __forceinline__ void slow_work(LaneState &L, const EntParams &P, const uint32_t *ctx,
-                                          const uint16_t *s_bend) {
-    if (L.st == S_EGS) {
-        // a suffix of more than 16 bits: the batched division form in pieces
-        // (src/mc_codec.c:219-224); magnitude 12 + x, x = (1 << nb | suffix) - 1
-        const uint32_t nb = L.rem;
-        const uint32_t m = 11u + ((1u << (nb & 31)) | bypass_long(L, nb));
-        L.rem = 0;
-        L.acc = 0;
-        if (m != 0) {   // the sign follows as a fast bypass bin
-            L.m = m;
-            L.st = F_BYP;
-            load_ctx(L, ctx);
-            return;
+// The rest of the coefficient at p - 1: for m > 12 the Exp-Golomb suffix of
+// m - 12 bits (the magnitude is 11 + (1 << nb | suffix), src/mc_codec.c:234-238,
+// 268-275), then sign and entry; false when the block ends (overflow pool
+// exhausted: corrupt streams only). The suffix of nb <= 16 bits is the
+// reference's batched read range >>= nb, q = min(code / range, 2^nb - 1),
+// code -= q * range: with the range's low nb bits cleared first, nb halvings
+// are that long division bit by bit, clamp included, and leave the same code
+// and range.
+__device__ __forceinline__ bool finish_coef(LaneState &L, const EntParams &P, uint32_t m) {
+    if (m > 12u) {
+        const uint32_t nb = m - 12u;
+        uint32_t acc = 1u << (nb & 31u);
+        if (nb <= 16u) {
+            uint32_t r = L.range & (0xFFFFFFFFu << nb);
+            acc = 1;
+            for (uint32_t i = 0; i < nb; ++i) {
+                r >>= 1;
+                const bool b = L.code >= r;
+                L.code = b ? L.code - r : L.code;
+                acc = 2u * acc + (b ? 1u : 0u);
+            }
+            L.range = r;
+            renorm(L);
+        } else {
+            acc |= bypass_long(L, nb);
         }
-        // m wrapped to 0 (a corrupt stream only): a zero-level coefficient,
-        // recorded here so that m == 0 keeps meaning "Exp-Golomb prefix"
-        bypass_bits(L, 1);
-        if (!put_entry(L, P, L.p)) return;
-        L.p++;
-        L.st = F_SIG;
-        L.k = 0;
-        if (L.p >= L.stop) position_event(L, ctx, s_bend);
-        else load_ctx(L, ctx);
+        m = 11u + acc;
+    }
+    const uint32_t neg = bypass_bits(L, 1);
+    return put_entry(L, P, (L.p - 1u) | ((neg ? 0u - m : m) << 16));
+}
+
+// The slow states of one lane, run while the rest of its warp waits.
+__device__ __forceinline__ void slow_work(LaneState &L, const EntParams &P, uint32_t *ctx, const uint16_t *s_bend) {
+    if (L.st == S_LAST) {
+        uint32_t k = 0;
+        while (k < 12 && ctx_bin(L, ctx + (kCtxMag + k) * 32)) ++k;
+        if (k == 12) {
+            while (bypass_bits(L, 1)) {
+                if (++k >= 12u + (uint32_t)kEgCap) { L.bad = 1; L.st = S_DONE; return; }
+            }
+        }
+        if (finish_coef(L, P, k < 12u ? k + 1u : k)) L.st = S_END;
         return;
     }
     // S_END
@@ -357,114 +381,132 @@ __device__ __forceinline__ void stg_if(bool pred, uint32_t *p, uint32_t v) {
     if (pred) *p = v;
 }
 
-// The rare events of a fast step, in this order: a window refill, the rest of
-// a renormalisation (none inside an Exp-Golomb suffix), an entry past the
-// block's arena share, the end of an Exp-Golomb prefix (a suffix of nb bits
-// follows: the range loses its low nb bits, which is the batched read's
-// range >> nb, and the suffix bits then halve it, or nb = 0 and the sign
-// follows), the end of a suffix (the magnitude is known; the sign follows),
-// and a scan position at a band change or the end of the scan.
-enum : uint32_t { EV_PFX = 1, EV_PFX_ONE = 2, EV_SFX = 4, EV_OVF = 8, EV_POS = 16 };
+// p + ((4096 - p) >> 4) and p - (p >> 4) (src/mc_codec.c:198-204) as one
+// multiply-add and a shift: equal for every p in 0..4096
+__device__ __forceinline__ uint32_t prob_after0(uint32_t p) { return (15u * p + 4096u) >> 4; }
+__device__ __forceinline__ uint32_t prob_after1(uint32_t p) { return (15u * p + 15u) >> 4; }
+
+// The rare events of a fast step: a coefficient that goes on in finish_coef
+// (an Exp-Golomb suffix, or a sign that the step had no bytes left for), a
+// prefix at its cap and an entry past the block's arena share (corrupt streams
+// only), and a scan position at a band change or the end of the scan.
+enum : uint32_t { EV_COEF = 1, EV_CAP = 2, EV_OVF = 4, EV_POS = 8 };
 __device__ __forceinline__ void fast_event(LaneState &L, const EntParams &P, const uint32_t *ctx,
                                            const uint16_t *s_bend, uint32_t why, uint32_t v) {
-    if (L.sel == kSel0 + 4) refill(L);
-    if (!(L.st == F_BYP && L.rem != 0)) renorm(L);
-    if ((why & EV_OVF) && !put_entry(L, P, v)) return;   // corrupt stream: pool exhausted, block ends
-    if (why & EV_PFX) {
-        if (why & EV_PFX_ONE) { L.bad = 1; L.st = S_DONE; return; }   // prefix cap reached (corrupt stream)
-        const uint32_t nb = L.k - kEgBase;                            // one-bits of the prefix
-        if (nb == 0) {
-            L.m = 12;
-        } else if (nb <= 16) {
-            L.rem = nb;
-            L.acc = 0;
-            L.range &= ~((1u << nb) - 1u);
-        } else {
-            L.rem = nb;
-            L.st = S_EGS;
-        }
-    }
-    if (why & EV_SFX) L.m = 11u + ((1u << (L.k - kEgBase)) | L.acc);
-    if (why & EV_POS) position_event(L, ctx, s_bend);
+    if ((why & EV_COEF) && !finish_coef(L, P, v >> 16)) return;
+    if (why & EV_CAP) { L.bad = 1; L.st = S_DONE; return; }
+    if ((why & EV_OVF) && !put_entry(L, P, v)) return;   // pool exhausted, block ends
+    if (L.p >= L.stop && L.k == 0) position_event(L, ctx, s_bend);
 }
 
-// One bin of every lane. The significance bin of position p uses context
-// band*4 + min(popcount(last 16 significance flags), 3) (src/mc_codec.c:249-259
-// and 353-375); magnitude rung k context 56+k (src/mc_codec.c:268-275); signs
-// and Exp-Golomb bits are bypass bins (:205, 216-238) computed by the same
-// instructions with r0 = range/2 and the scratch context slot. An Exp-Golomb
-// suffix of nb <= 16 bits is the reference's batched read range >>= nb,
-// q = min(code / range, 2^nb - 1), code -= q * range: with the range's low nb
-// bits cleared first, nb halvings without renormalisation between them are
-// that long division bit by bit, clamp included, and leave the same code and
-// range; the renormalisation follows the last bit.
-// The step is software-pipelined: the bin's context value (pc, slot cc) was
-// fetched during the previous step, and this step fetches both candidate
-// contexts of the next bin (one per value of this bin) before it decodes, so
-// the shared-memory round trip overlaps the arithmetic; a next context equal
-// to this bin's takes the freshly updated value instead. Every lane runs the
-// same straight-line code of selects and predicated stores; a parked lane
-// passes through unchanged, and lanes in slow states never get here. Rare
-// events (see fast_event) share one branch.
-__device__ __forceinline__ void fast_step(LaneState &L, const EntParams &P, uint32_t *ctx, const uint16_t *s_bend) {
-    const uint32_t st = L.st, m0 = L.m, rem0 = L.rem, k0 = L.k, cc = L.cc, pc = L.pc;
-    const bool is_sig = st == F_SIG, is_mag = st == F_MAG, is_byp = st == F_BYP;
-    const bool is_sign = is_byp & (m0 != 0u);
-    const bool is_sfx = is_byp & (rem0 != 0u);
-    const bool is_pfx = is_byp & !is_sign & !is_sfx;
-    // candidate contexts of the next bin: c0 if this bin is 0, c1 if it is 1.
-    // After a significance bin of 0 the flag window drops its oldest flag.
-    const uint32_t csig = L.sigb + min((uint32_t)__popc(L.hist & (is_sig ? 0x7FFFu : 0xFFFFu)), 3u);
-    const uint32_t c0 = (is_sig | is_sign) ? csig : kScr;
-    const uint32_t c1 = is_sig ? (uint32_t)kCtxMag : (is_mag ? min(cc + 1u, kScr) : c0);
-    const uint32_t q0 = ctx[c0 * 32];
-    const uint32_t q1 = ctx[c1 * 32];
-    // this bin
-    const uint32_t r0 = is_byp ? L.range >> 1 : (L.range >> 12) * pc;
-    const bool bit = L.code >= r0;
-    const uint32_t code = bit ? L.code - r0 : L.code;
-    const uint32_t range = (bit & !is_byp) ? L.range - r0 : r0;
-    const uint32_t np0 = (15u * pc + (bit ? 15u : 4096u)) >> 4;   // p - (p >> 4) or p + ((4096 - p) >> 4)
-    ctx[cc * 32] = np0;   // bypass bins write the scratch slot
-    // renormalisation, first byte (src/mc_codec.c:202); not between the bits
-    // of a suffix
-    const bool sup = is_sfx & (rem0 > 1u);
-    const bool need = (range < (1u << 24)) & !sup;
-    L.code = need ? __byte_perm(code, L.w, L.sel) : code;
-    L.range = need ? range << 8 : range;
-    L.sel += need ? 1u : 0u;
-    // next bin's context
-    const uint32_t ncc = bit ? c1 : c0;
-    L.pc = ncc == cc ? np0 : (bit ? q1 : q0);
-    L.cc = ncc;
-    // state
-    const bool esc = is_mag & bit & (k0 == 11u);   // 12th rung set: Exp-Golomb tail
-    L.hist = is_sig ? (L.hist << 1) | (bit ? 1u : 0u) : L.hist;
-    L.k = is_sig ? 0u : ((bit & !is_sfx) ? k0 + 1u : k0);
-    L.m = (is_mag & !bit) ? k0 + 1u : (is_sign ? 0u : m0);
-    L.acc = is_sfx ? (L.acc << 1) | (bit ? 1u : 0u) : L.acc;
-    L.rem = is_sfx ? rem0 - 1u : rem0;
-    L.st = is_sig ? (bit ? (uint32_t)F_MAG : (uint32_t)F_SIG)
-                  : (is_mag ? ((bit & !esc) ? (uint32_t)F_MAG : (uint32_t)F_BYP) : (is_sign ? (uint32_t)F_SIG : st));
-    // a sign completes the coefficient at scan position p: its entry
-    const uint32_t p = L.p;
-    const bool adv = (is_sig & !bit) | is_sign;
-    const uint32_t np = p + (adv ? 1u : 0u);
-    L.p = np;
-    const uint32_t v = p | ((bit ? 0u - m0 : m0) << 16);
-    const bool room = L.nent < L.cap;
-    stg_if(is_sign & room, L.ent + L.nent, v);
-    L.nent += (is_sign & room) ? 1u : 0u;
-    const bool pfx_end = is_pfx & (!bit | (k0 + 1u >= kEgBase + (uint32_t)kEgCap));
-    const bool pos = adv & (np >= L.stop);
-    const bool ovf = is_sign & !room;
-    const bool sfx_end = is_sfx & (rem0 == 1u);
-    if ((L.sel == kSel0 + 4) | ((L.range < (1u << 24)) & !sup) | pfx_end | sfx_end | pos | ovf) {
-        const uint32_t why = (pfx_end ? (uint32_t)EV_PFX : 0u) | ((pfx_end & bit) ? (uint32_t)EV_PFX_ONE : 0u) |
-                             (sfx_end ? (uint32_t)EV_SFX : 0u) | (ovf ? (uint32_t)EV_OVF : 0u) |
-                             (pos ? (uint32_t)EV_POS : 0u);
-        fast_event(L, P, ctx, s_bend, why, v);
+// Bits that a renormalisation shifts in (src/mc_codec.c:202): two bytes at
+// most, since the range is at least 2^24 before a bin and a split leaves at
+// least 15 * 2^12 of it (p <= 4081 once adapted).
+__device__ __forceinline__ uint32_t renorm_bits(uint32_t range) {
+    return range < (1u << 16) ? 16u : (range < kTop ? 8u : 0u);
+}
+
+// One step of every lane: up to a whole coefficient, by the same straight-line
+// code of selects and predicated accesses for every lane.
+//  1. A lane at a significance bin first takes a run of one or four
+//     insignificant positions. While bins are 0 the code does not change and
+//     the range only falls, so a run needs no compare per bin: its last split
+//     above both the code and the renormalisation bound (one compare with the
+//     larger) says that all its bins are 0 and none renormalises. Its length
+//     leaves room for a bin in the same context after it.
+//  2. Then one significance bin (src/mc_codec.c:353-375).
+//  3. A significant position goes on with magnitude rung 0 at once, a lane at
+//     a later rung or in an Exp-Golomb prefix with its next bin
+//     (src/mc_codec.c:268-275).
+//  4. A magnitude that closes takes its sign at once (:205).
+// A lane without a bin of a kind keeps its range by splitting at the range
+// itself. The context values come from shared memory a step ahead (ps, pm):
+// loaded as soon as the next position's density class and the next rung are
+// known, after the store of the context just used.
+// One step reads at most 40 bits (see renorm_bits), the window always holds
+// at least 40, and the 32 extracted here serve all but a sign after more than
+// 24 bits, which is left to fast_event. Returns the events of the lane; v is
+// its entry (for EV_COEF, the argument of finish_coef in the high half).
+// What bounds it: integer issue, most of it on the ALU pipe at half rate. Runs
+// of length 1 or 4: allowing 1 to 4 takes 5 % fewer steps (of a q=6 sample: 424
+// against 445, 1028 without runs) of a tenth more instructions. A step of one
+// bin per lane took 2041 steps a block at q=6 and 9870 at q=1; 64 chunks at
+// q=6: 2.68 ms with it, 1.54 ms with this one.
+__device__ __forceinline__ uint32_t fast_step(LaneState &L, const EntParams &P, uint32_t *ctx, uint32_t &v) {
+    const uint32_t k0 = L.k;
+    const bool is_sig = k0 == 0u;
+    uint32_t code = L.code, range = L.range, pr = L.ps, p = L.p;
+    uint32_t x = funnel_left(L.w2, L.w, L.used);   // the next 32 payload bits
+    // 1. zeros
+    {
+        const uint32_t floor1 = code >= kTop ? code : kTop - 1u;
+        const uint32_t room = is_sig ? L.lim - p : 0u;   // > 0 at a significance bin
+        const uint32_t r1 = (range >> 12) * pr, q1 = prob_after0(pr);
+        const uint32_t r2 = (r1 >> 12) * q1, q2 = prob_after0(q1);
+        const uint32_t r3 = (r2 >> 12) * q2, q3 = prob_after0(q2);
+        const uint32_t r4 = (r3 >> 12) * q3, q4 = prob_after0(q3);
+        const bool z1 = (r1 > floor1) & (room > 1u), z4 = (r4 > floor1) & (room > 4u);
+        range = z4 ? r4 : (z1 ? r1 : range);
+        pr = z4 ? q4 : (z1 ? q1 : pr);
+        p += z4 ? 4u : (z1 ? 1u : 0u);
     }
+    // 2. one significance bin
+    const uint32_t r1 = is_sig ? (range >> 12) * pr : range;
+    const bool one = is_sig & (code >= r1);
+    code = one ? code - r1 : code;
+    range = one ? range - r1 : r1;
+    pr = (15u * pr + (one ? 15u : 4096u)) >> 4;
+    if (is_sig) ctx[L.cs * 32] = pr;
+    const uint32_t s1 = renorm_bits(range);
+    code = funnel_left(x, code, s1);
+    x <<= s1;
+    range <<= s1;
+    // the next position, its density class and context
+    p += is_sig ? 1u : 0u;
+    L.p = p;
+    L.e3 = one ? L.e2 : L.e3;
+    L.e2 = one ? L.e1 : L.e2;
+    L.e1 = one ? p + 16u : L.e1;
+    density(L);
+    L.ps = ctx[L.cs * 32];
+    // 3. one magnitude rung
+    const bool act = one | !is_sig;
+    const uint32_t pm = L.pm;
+    const bool pfx = k0 >= 12u;
+    const uint32_t r2 = act ? (range >> (pfx ? 1u : 12u)) * pm : range;
+    const bool up = act & (code >= r2);
+    code = up ? code - r2 : code;
+    range = up & !pfx ? range - r2 : r2;   // a bypass bin leaves the half either way
+    uint32_t *cm = ctx + (kCtxMag + k0) * 32;
+    if (act & !pfx) *cm = (15u * pm + (up ? 15u : 4096u)) >> 4;
+    const uint32_t kn = up ? k0 + 1u : 0u;
+    L.k = kn;
+    L.pm = ctx[(kCtxMag + min(kn, 12u)) * 32];   // the next rung's
+    const uint32_t s2 = renorm_bits(range);
+    code = funnel_left(x, code, s2);
+    x <<= s2;
+    range <<= s2;
+    // 4. the sign of a magnitude that closed, and the entry of the coefficient at p - 1
+    const bool closed = act & !up;
+    const bool sign = closed & (k0 <= 12u) & (s1 + s2 <= 24u);
+    const uint32_t r3 = sign ? range >> 1 : range;
+    const bool neg = sign & (code >= r3);
+    code = neg ? code - r3 : code;
+    const uint32_t s3 = r3 < kTop ? 8u : 0u;
+    L.code = funnel_left(x, code, s3);
+    L.range = r3 << s3;
+    const uint32_t m = pfx ? k0 : k0 + 1u;
+    v = (p - 1u) | ((neg ? 0u - m : m) << 16);
+    const bool room_e = L.nent < L.cap;
+    stg_if(sign & room_e, L.ent + L.nent, v);
+    L.nent += (sign & room_e) ? 1u : 0u;
+    // the window
+    const uint32_t u = L.used + s1 + s2 + s3;
+    L.used = u;
+    if (u >= 32u) refill(L);
+    return ((closed & !sign) ? (uint32_t)EV_COEF : 0u) |
+           ((kn >= 12u + (uint32_t)kEgCap) ? (uint32_t)EV_CAP : 0u) |
+           ((sign & !room_e) ? (uint32_t)EV_OVF : 0u) | (((kn == 0u) & (p >= L.stop)) ? (uint32_t)EV_POS : 0u);
 }
 
 // Work queue of a launch: the first ncoded entries of the processing order
@@ -484,13 +526,12 @@ __device__ __forceinline__ int claim_next(Claim &c, const EntParams &P, int nlan
 
 // Every lane of the warp decodes blocks until the queue is empty. Lane gtid
 // starts with entry gtid (none when gtid < 0), then claims from the counter. Fast steps
-// run while every lane is in a fast state or parked; when a lane reaches a
-// slow state the warp leaves the loop, that lane works its slow states off
-// (finishing its block and starting the next one), and the loop resumes.
-// Every block ends after a bounded number of bins (finite scan, capped
-// Exp-Golomb prefixes, bounded correction count) and every lane claims at
-// most ncoded blocks, so the loop ends. on_done(item) runs for every
-// finished block.
+// run while every lane runs or is parked; when a lane reaches a slow state the
+// warp leaves the loop, that lane works its slow states off (finishing its
+// block and starting the next one), and the loop resumes. Every block ends
+// after a bounded number of bins (finite scan, capped Exp-Golomb prefixes,
+// bounded correction count) and every lane claims at most ncoded blocks, so
+// the loop ends. on_done(item) runs for every finished block.
 template <class OnDone>
 __device__ __forceinline__ void run_lanes(LaneState &L, const EntParams &P, uint32_t *ctx, const uint16_t *s_bend,
                                           int gtid, int nlanes, OnDone on_done) {
@@ -499,15 +540,7 @@ __device__ __forceinline__ void run_lanes(LaneState &L, const EntParams &P, uint
     L.st = S_DONE;
     Claim c = gtid >= 0 ? Claim{gtid, gtid + 1} : Claim{0, 0};   // gtid < 0: queue claims only
     for (;;) {
-        // two steps per loop turn (the loop-carried lane state then needs
-        // no register shuffling between the two), the check after each
-        for (;;) {
-            if (__any_sync(0xFFFFFFFFu, L.st >= S_END)) break;
-            fast_step(L, P, ctx, s_bend);
-            if (__any_sync(0xFFFFFFFFu, L.st >= S_END)) break;
-            fast_step(L, P, ctx, s_bend);
-        }
-        while (L.st >= S_END) {
+        while (L.st >= S_LAST) {
             if (L.st != S_DONE) {
                 slow_work(L, P, ctx, s_bend);
                 continue;
@@ -521,6 +554,14 @@ __device__ __forceinline__ void run_lanes(LaneState &L, const EntParams &P, uint
             else park(L);
         }
         if (__all_sync(0xFFFFFFFFu, L.st == S_IDLE)) break;
+        for (;;) {
+            uint32_t v;
+            const uint32_t why = fast_step(L, P, ctx, v);
+            if (__any_sync(0xFFFFFFFFu, why != 0)) {
+                if (why) fast_event(L, P, ctx, s_bend, why, v);
+                if (__any_sync(0xFFFFFFFFu, L.st >= S_LAST)) break;
+            }
+        }
     }
 }
 
@@ -528,25 +569,42 @@ __device__ __forceinline__ void run_lanes(LaneState &L, const EntParams &P, uint
 // the latency of one thread alone on its warp (no other lane shares its
 // instructions). All contexts of the coefficient loop that the common bins
 // use are held in registers: the four significance contexts of the current
-// band (the one in use as a live probability, written back when the density
-// changes) and the twelve magnitude rungs. A run of insignificant positions
-// then costs per bin the range split, the compare, the probability update
-// and one test for the rare events (a renormalisation, the flag that leaves
-// the 16-position density window, the end of the band or the scan). A
-// significant bin decodes its coefficient (magnitude, sign, entry) in place
-// and the run goes on; the common steps of a coefficient use selects rather
-// than branches, whose divergence bookkeeping costs more than their work.
-// Band changes, Exp-Golomb tails and the corrections take the shared step
-// functions (position_event, renorm, eg_value, put_entry, slow_work). Bands
-// only advance, so a band's register contexts are never written back to
-// shared memory, and the magnitude rungs are used by nothing else.
-__device__ __forceinline__ uint32_t pick4(uint32_t c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
-    return c == 0 ? a0 : (c == 1 ? a1 : (c == 2 ? a2 : a3));
+// band and the twelve magnitude rungs. Bands only advance, so a band's
+// register contexts are never written back to shared memory, and the magnitude
+// rungs are used by nothing else. The common steps use selects rather than
+// branches, whose divergence bookkeeping costs more than their work.
+// Two loops take the significance bins. Where three or more of the last 16
+// positions were significant (density class 3), half of the positions are, and
+// the loop takes one bin at a time, its probability in the class's own
+// register. In the sparser classes runs of zeros are long and go four at a
+// time: while bins are 0 the code does not change and the range only falls, so
+// four splits are computed straight through and one compare of the last with
+// the code and the renormalisation bound decides them all.
+// Band changes and the corrections take the shared step functions
+// (position_event, put_entry, slow_work).
+
+// Renormalisation with the common case (one byte) by selects; a second byte
+// or a window refill takes the loop.
+__device__ __forceinline__ void renorm_sel(LaneState &L) {
+    const uint32_t s = L.range < kTop ? 8u : 0u;
+    L.code = funnel_left(L.w << L.used, L.code, s);
+    L.range <<= s;
+    L.used += s;
+    if ((L.used == 32u) | (L.range < kTop)) {
+        if (L.used == 32u) refill(L);
+        renorm(L);
+    }
 }
-// p + ((4096 - p) >> 4) and p - (p >> 4) (src/mc_codec.c:198-204) as one
-// multiply-add and a shift: equal for every p in 0..4096
-__device__ __forceinline__ uint32_t prob_after0(uint32_t p) { return (15u * p + 4096u) >> 4; }
-__device__ __forceinline__ uint32_t prob_after1(uint32_t p) { return (15u * p + 15u) >> 4; }
+// One adaptive bin on a register context.
+__device__ __forceinline__ bool reg_bin(LaneState &L, uint32_t &g) {
+    const uint32_t r = (L.range >> 12) * g;
+    const bool b = L.code >= r;
+    L.code = b ? L.code - r : L.code;
+    L.range = b ? L.range - r : r;
+    g = (15u * g + (b ? 15u : 4096u)) >> 4;
+    renorm_sel(L);
+    return b;
+}
 // One magnitude rung on a register context; after a 1 the range is
 // renormalised here, after the closing 0 by the caller.
 __device__ __forceinline__ bool rung(LaneState &L, uint32_t &g) {
@@ -559,21 +617,16 @@ __device__ __forceinline__ bool rung(LaneState &L, uint32_t &g) {
     L.code -= r;
     L.range -= r;
     g = prob_after1(g);
-    if (L.range < (1u << 24)) renorm(L);
+    if (L.range < kTop) renorm(L);
     return true;
 }
-
-// Renormalisation with the common case (one byte, the window not emptied)
-// by selects; a second byte or a window refill takes the loop.
-__device__ __forceinline__ void renorm_sel(LaneState &L) {
-    const bool need = L.range < (1u << 24);
-    L.code = need ? __byte_perm(L.code, L.w, L.sel) : L.code;
-    L.range = need ? L.range << 8 : L.range;
-    L.sel += need ? 1u : 0u;
-    if ((L.sel == kSel0 + 4) | (L.range < (1u << 24))) {
-        if (L.sel == kSel0 + 4) refill(L);
-        renorm(L);
-    }
+// One bypass bin (src/mc_codec.c:205).
+__device__ __forceinline__ bool reg_bypass(LaneState &L) {
+    L.range >>= 1;
+    const bool b = L.code >= L.range;
+    L.code = b ? L.code - L.range : L.code;
+    renorm_sel(L);
+    return b;
 }
 
 __device__ __forceinline__ void solo_entropy(LaneState &L, const EntParams &P, uint32_t *ctx,
@@ -585,115 +638,99 @@ __device__ __forceinline__ void solo_entropy(LaneState &L, const EntParams &P, u
     uint32_t g3 = ctx[(kCtxMag + 3) * 32], g4 = ctx[(kCtxMag + 4) * 32], g5 = ctx[(kCtxMag + 5) * 32];
     uint32_t g6 = ctx[(kCtxMag + 6) * 32], g7 = ctx[(kCtxMag + 7) * 32], g8 = ctx[(kCtxMag + 8) * 32];
     uint32_t g9 = ctx[(kCtxMag + 9) * 32], g10 = ctx[(kCtxMag + 10) * 32], g11 = ctx[(kCtxMag + 11) * 32];
-    uint32_t h = L.hist & 0xFFFFu;   // the last 16 significance flags, newest in bit 0
-    uint32_t cnt = __popc(h);
-    // a position event; the band's contexts come into registers when it changes
-    auto event = [&]() {
-        L.hist = h;
-        position_event(L, ctx, s_bend);
-        if (L.sigb != sigb) {
-            sigb = L.sigb;
-            s0 = ctx[(sigb + 0) * 32]; s1 = ctx[(sigb + 1) * 32];
-            s2 = ctx[(sigb + 2) * 32]; s3 = ctx[(sigb + 3) * 32];
-        }
-        h = L.hist & 0xFFFFu;
-        cnt = __popc(h);
-    };
-    // the coefficient at L.p, known significant: the unary magnitude
-    // (src/mc_codec.c:268-275), the sign, the entry, the next position;
-    // false when the block ends (an Exp-Golomb prefix at the cap or the
-    // overflow pool exhausted: corrupt streams only)
-    auto coef = [&]() -> bool {
-        uint32_t m;
-        const uint32_t r = (L.range >> 12) * g0;   // rung 0, by selects
-        const bool b0 = L.code >= r;
-        L.code = b0 ? L.code - r : L.code;
-        L.range = b0 ? L.range - r : r;
-        g0 = (15u * g0 + (b0 ? 15u : 4096u)) >> 4;
-        renorm_sel(L);
-        if (!b0) {
-            m = 1;
-        } else {
-            if (!rung(L, g1)) m = 2;
-            else if (!rung(L, g2)) m = 3;
-            else if (!rung(L, g3)) m = 4;
-            else if (!rung(L, g4)) m = 5;
-            else if (!rung(L, g5)) m = 6;
-            else if (!rung(L, g6)) m = 7;
-            else if (!rung(L, g7)) m = 8;
-            else if (!rung(L, g8)) m = 9;
-            else if (!rung(L, g9)) m = 10;
-            else if (!rung(L, g10)) m = 11;
-            else if (!rung(L, g11)) m = 12;
-            else m = 0;
-            if (m == 0) {   // the twelfth rung set: 12 + an Exp-Golomb value
-                m = 12u + eg_value(L);
-                if (L.bad) { L.st = S_DONE; return false; }   // prefix cap
-            }
-            renorm(L);
-        }
-        L.range >>= 1;   // the sign, a bypass bin (src/mc_codec.c:205)
-        const bool neg = L.code >= L.range;
-        L.code = neg ? L.code - L.range : L.code;
-        renorm_sel(L);
-        const uint32_t v = L.p | ((neg ? 0u - m : m) << 16);
-        if (L.nent < L.cap) {
-            L.ent[L.nent++] = v;
-        } else if (!put_entry(L, P, v)) {
-            return false;   // S_DONE
-        }
-        ++L.p;
-        L.st = F_SIG;
-        if (L.p >= L.stop) event();
-        return true;
-    };
-    for (;;) {
-        if (L.st == F_MAG) {   // the implicit last position (lane_begin or an event)
-            if (!coef()) break;
-            continue;
-        }
-        if (L.st != F_SIG) break;
-        // a run of significance bins at L.p < L.stop, the context in use as
-        // the live probability pc
-        uint32_t c = min(cnt, 3u);
-        uint32_t pc = pick4(c, s0, s1, s2, s3);
-        for (;;) {
-            const uint32_t r0 = (L.range >> 12) * pc;
-            if (L.code >= r0) {   // significant
-                L.code -= r0;
-                L.range -= r0;
-                pc = prob_after1(pc);
-                s0 = c == 0 ? pc : s0; s1 = c == 1 ? pc : s1;
-                s2 = c == 2 ? pc : s2; s3 = c == 3 ? pc : s3;
-                h = (h << 1) | 1u;
-                cnt += 1u - (h >> 16);   // the flag that entered, the one that left
-                h &= 0xFFFFu;
-                renorm_sel(L);
-                if (!coef()) break;
-                if (L.st != F_SIG) break;
-                c = min(cnt, 3u);
-                pc = pick4(c, s0, s1, s2, s3);
-                continue;
-            }
-            L.range = r0;
-            pc = prob_after0(pc);
-            h <<= 1;
-            ++L.p;
-            if ((L.range < (1u << 24)) | (L.p >= L.stop) | (h > 0xFFFFu)) {
-                if (L.range < (1u << 24)) renorm(L);
-                if ((L.p >= L.stop) | (h > 0xFFFFu)) {
-                    s0 = c == 0 ? pc : s0; s1 = c == 1 ? pc : s1;
-                    s2 = c == 2 ? pc : s2; s3 = c == 3 ? pc : s3;
-                    cnt -= h >> 16;   // the flag that left the window
-                    h &= 0xFFFFu;
-                    if (L.p >= L.stop) {
-                        event();
-                        if (L.st != F_SIG) break;
+    bool one = L.st == S_LAST;   // the position at p - 1 is significant, its coefficient is next
+    bool more = L.st <= S_LAST;
+    while (more) {
+        if (!one) {
+            if (L.p < L.e3) {   // density class 3
+                const uint32_t end = min(L.stop, L.e3);
+                for (;;) {
+                    const uint32_t r = (L.range >> 12) * s3;
+                    if (L.code >= r) {   // significant
+                        L.code -= r;
+                        L.range -= r;
+                        s3 = prob_after1(s3);
+                        ++L.p;
+                        renorm_sel(L);
+                        one = true;
+                        break;
                     }
-                    c = min(cnt, 3u);
-                    pc = pick4(c, s0, s1, s2, s3);
+                    L.range = r;
+                    s3 = prob_after0(s3);
+                    ++L.p;
+                    if ((r < kTop) | (L.p >= end)) {
+                        if (r < kTop) renorm(L);
+                        if (L.p >= end) break;
+                    }
                 }
+            } else {
+                const bool a2 = L.p < L.e2, a1 = L.p < L.e1;
+                const uint32_t end = min(L.stop, a2 ? L.e2 : (a1 ? L.e1 : 0xFFFFFFFFu));
+                uint32_t pc = a2 ? s2 : (a1 ? s1 : s0);
+                do {
+                    const uint32_t floor1 = L.code >= kTop ? L.code : kTop - 1u;
+                    while (L.p + 4u <= end) {
+                        const uint32_t r1 = (L.range >> 12) * pc, q1 = prob_after0(pc);
+                        const uint32_t r2 = (r1 >> 12) * q1, q2 = prob_after0(q1);
+                        const uint32_t r3 = (r2 >> 12) * q2, q3 = prob_after0(q2);
+                        const uint32_t r4 = (r3 >> 12) * q3;
+                        if (r4 <= floor1) break;
+                        L.range = r4;
+                        pc = prob_after0(q3);
+                        L.p += 4;
+                    }
+                    if (L.p >= end) break;
+                    one = reg_bin(L, pc);
+                    ++L.p;
+                } while (!one & (L.p < end));
+                s0 = a1 ? s0 : pc;
+                s1 = a1 & !a2 ? pc : s1;
+                s2 = a2 ? pc : s2;
             }
+            if (one) {
+                L.e3 = L.e2;
+                L.e2 = L.e1;
+                L.e1 = L.p + 16u;
+            }
+        }
+        if (one) {
+            // the coefficient at p - 1: the unary magnitude
+            // (src/mc_codec.c:268-275), the sign, the entry
+            uint32_t m = 1;
+            if (reg_bin(L, g0)) {
+                if (!rung(L, g1)) m = 2;
+                else if (!rung(L, g2)) m = 3;
+                else if (!rung(L, g3)) m = 4;
+                else if (!rung(L, g4)) m = 5;
+                else if (!rung(L, g5)) m = 6;
+                else if (!rung(L, g6)) m = 7;
+                else if (!rung(L, g7)) m = 8;
+                else if (!rung(L, g8)) m = 9;
+                else if (!rung(L, g9)) m = 10;
+                else if (!rung(L, g10)) m = 11;
+                else if (!rung(L, g11)) m = 12;
+                else {   // the twelfth rung set: 12 + an Exp-Golomb value
+                    m = 12u + eg_value(L);
+                    if (L.bad) { L.st = S_DONE; break; }   // prefix cap (corrupt streams only)
+                }
+                renorm(L);
+            }
+            const bool neg = reg_bypass(L);
+            const uint32_t v = (L.p - 1u) | ((neg ? 0u - m : m) << 16);
+            if (L.nent < L.cap) L.ent[L.nent++] = v;
+            else if (!put_entry(L, P, v)) break;   // overflow pool exhausted (corrupt streams only)
+            L.st = F_RUN;
+            one = false;
+        }
+        if (L.p >= L.stop) {   // the band's contexts come into registers when it changes
+            position_event(L, ctx, s_bend);
+            if (L.sigb != sigb) {
+                sigb = L.sigb;
+                s0 = ctx[(sigb + 0) * 32]; s1 = ctx[(sigb + 1) * 32];
+                s2 = ctx[(sigb + 2) * 32]; s3 = ctx[(sigb + 3) * 32];
+            }
+            one = L.st == S_LAST;
+            more = L.st <= S_LAST;
         }
     }
     while (L.st != S_DONE) slow_work(L, P, ctx, s_bend);
@@ -1378,13 +1415,8 @@ __global__ void __launch_bounds__(128) k_fused_tail(FusedParams F) {
 // The single-block calls (mc_archive_decode_block, mc_dec_block): one CTA
 // decodes one block end to end in one launch, with the work item as a kernel
 // argument -- no batch layout, no host-to-device copies, no second launch.
-// Thread 0 runs the entropy decode through the k_entropy step functions
-// (fast_step, slow_work for the rare states), the CTA then reconstructs
-// the block. A branchy scalar loop over the same states was measured slower
-// per bin (p99 block latency 1.23 ms against 0.93): each bin's shared-memory
-// context load and branch resolution then sit on the serial chain, which the
-// warp step avoids by fetching both candidate contexts ahead, without
-// branches.
+// Thread 0 runs the entropy decode (solo_entropy), the CTA then reconstructs
+// the block.
 
 static_assert(sizeof(DecItem) % 16 == 0, "SoloScratch::hdr must sit on a 16-byte boundary");
 
@@ -1506,12 +1538,18 @@ static cudaError_t launch_entropy_w(const EntParams &p, int ctas_per_sm, cudaStr
 }
 
 // The single-thread share when a launch configuration leaves it open, from
-// the launch's coded blocks (q=6 batches on a B200): up to about 10 chunks'
-// worth every block on a single thread (its time is the longest block's
-// chain, a few times shorter there), up to about 30 chunks' worth the longest
-// 1/64, beyond that none (a lane of 32 issues fewer instructions per bin).
-constexpr int kSoloAllMax = 28 * 1024, kSoloShareMax = 90 * 1024;
-static int auto_solo(int ncoded) { return ncoded <= kSoloAllMax ? 1 : (ncoded <= kSoloShareMax ? 64 : 0); }
+// the launch's coded blocks. Below about 4 chunks' worth the stage's time is the
+// longest block's chain, which a single thread runs fastest (q=6: 2 chunks 530
+// us against 723 with lanes alone, 4 chunks 584 against 745; q=12: 281 against
+// 391). Up to about 60 chunks' worth the longest blocks, four for each SM (one
+// for each of its schedulers), run on single threads beside the lanes (8 chunks
+// 643 us against 764 with lanes alone and 1042 on single threads; 16: 762 / 848
+// / 2087; 48: 1250 / 1333); a full 64 chunks gain nothing (1548 / 1554).
+constexpr int kSoloAllMax = 15 * 1024, kSoloShareMax = 200 * 1024;
+static int auto_solo(int ncoded) {
+    if (ncoded <= kSoloAllMax) return 1;
+    return ncoded <= kSoloShareMax ? ncoded / (4 * num_sms()) : 0;
+}
 
 cudaError_t launch_entropy(const EntParams &p, const LaunchCfg &cfg, cudaStream_t s) {
     if (p.ncoded <= 0) return cudaSuccess;

@@ -18,6 +18,15 @@
 
 namespace mcb {
 
+// The high word of (hi:lo) shifted left by s, 0 <= s < 32.
+MCB_HD inline uint32_t funnel_left(uint32_t lo, uint32_t hi, uint32_t s) {
+#if defined(__CUDA_ARCH__)
+    return __funnelshift_l(lo, hi, s);
+#else
+    return s ? (hi << s) | (lo >> (32 - s)) : hi;
+#endif
+}
+
 constexpr int kBlk = 16;            // block edge (voxels)
 constexpr int kN3 = 4096;           // voxels per block
 constexpr int kChunk = 256;         // chunk edge (voxels)
