@@ -13,7 +13,7 @@
 // conflict-free). Output per block: a small header (dc, flags) and a list of
 // nonzero levels plus corrections.
 //
-// Stage 2, k_reconstruct: one CTA (128 threads) per block. Dequantise into a
+// Stage 2, k_reconstruct: one CTA (64 threads) per block. Dequantise into a
 // dense coefficient box bounded by the block's extents, then the three
 // separable DCT-III passes along x, y, z, each output accumulated over
 // ascending k in single precision with explicit round-to-nearest adds and
@@ -34,6 +34,8 @@
 namespace mcb {
 
 __constant__ float c_cos[16][16];
+// {c[k][m], c[k][m], c[k][m+1], c[k][m+1]} at [k][m/2]: weights of packed pairs
+__constant__ float4 c_cos2[16][8];
 // c_bend[b]: the first scan position past band b (b < 7), then kN3 and a
 // sentinel; kernels copy it into shared memory at start
 __constant__ uint16_t c_bend[9];
@@ -1168,16 +1170,29 @@ __device__ __forceinline__ void reconstruct_block(const RecParams &P, int item, 
     __syncthreads();
 }
 
-// Clipped store of one staged block: one 16-voxel row per thread step.
-__device__ __forceinline__ void store_block(const DecItem &it, const uint8_t *stage) {
+struct StageRows {   // z slices of kStageZ bytes
+    const uint8_t *p;
+    __device__ const uint8_t *operator()(int z, int y) const { return p + z * kStageZ + y * 16; }
+};
+// Clipped store of one staged block (row (z, y) at stage_row(z, y)) by nthr
+// threads, this one thread `tid` of them: one 16-voxel row per thread step.
+template <class Row>
+__device__ __forceinline__ void store_block(const DecItem &it, Row stage_row, int tid, int nthr) {
+    uint8_t *dst = reinterpret_cast<uint8_t *>(it.dst);
+    if (it.clip_lo == kClipFullLo && it.clip_hi == kClipFullHi) {
+        for (int r = tid; r < 256; r += nthr) {
+            const int z = r >> 4, y = r & 15;
+            store_row16(dst + z * it.sz + y * it.sy, *reinterpret_cast<const uint4 *>(stage_row(z, y)));
+        }
+        return;
+    }
     const int z0 = it.clip_lo >> 8, y0 = (it.clip_lo >> 4) & 15, x0 = it.clip_lo & 15;
     const int z1 = it.clip_hi >> 8, y1 = (it.clip_hi >> 4) & 15, x1 = it.clip_hi & 15;
     const int ny = y1 - y0 + 1, nrows = (z1 - z0 + 1) * ny;
-    uint8_t *dst = reinterpret_cast<uint8_t *>(it.dst);
-    for (int r = threadIdx.x; r < nrows; r += blockDim.x) {
+    for (int r = tid; r < nrows; r += nthr) {
         const int z = z0 + r / ny, y = y0 + r % ny;
         uint8_t *row = dst + z * it.sz + y * it.sy;
-        const uint8_t *srow = stage + z * kStageZ + y * 16;
+        const uint8_t *srow = stage_row(z, y);
         if (x0 == 0 && x1 == 15) {
             store_row16(row, *reinterpret_cast<const uint4 *>(srow));
         } else {
@@ -1195,48 +1210,349 @@ __device__ __forceinline__ bool pairable(const DecItem &a, const DecItem &b) {
            (a.sy & 31) == 0 && (a.sz & 31) == 0;
 }
 
-__global__ void __launch_bounds__(128, 5) k_reconstruct(RecParams P) {
-    // sA: pass-1 output, then the second block's stage; sB: coefficient box,
-    // then pass-2 output; sStage0: the first block's stage
-    __shared__ __align__(16) float sA[16 * 16 * kRowF];
-    __shared__ __align__(16) float sB[kBoxB];
-    __shared__ __align__(16) uint8_t sStage0[kStageBytes];
-    __shared__ __align__(16) float4 sW[16 * 8];   // [k][m/2] = {c[k][m], c[k][m], c[k][m+1], c[k][m+1]}
-    uint8_t *const sStage1 = reinterpret_cast<uint8_t *>(sA);
-    for (int i = threadIdx.x; i < 16 * 8; i += blockDim.x) {
-        const int k = i >> 3, mm = (i & 7) * 2;
-        sW[i] = make_float4(c_cos[k][mm], c_cos[k][mm], c_cos[k][mm + 1], c_cos[k][mm + 1]);
-    }
-    rec_init(sB);
-    __syncthreads();
-    const int tid = threadIdx.x;
-    const int npairs = (P.n + 1) / 2;
-    for (int pr = blockIdx.x; pr < npairs; pr += gridDim.x) {
-        const int j0 = 2 * pr, j1 = 2 * pr + 1;
-        const int i0 = P.idx ? (int)P.idx[j0] : j0;
-        const int i1 = j1 < P.n ? (P.idx ? (int)P.idx[j1] : j1) : -1;
-        const int jn = 2 * (pr + gridDim.x);   // this CTA's next pair
-        const int in = jn < P.n ? (P.idx ? (int)P.idx[jn] : jn) : -1;
-        reconstruct_block<false>(P, i0, sA, sB, sStage0, sW, i1 >= 0 ? i1 : in);
-        const DecItem a = P.items[i0];
-        if (i1 >= 0) {
-            reconstruct_block<false>(P, i1, sA, sB, sStage1, sW, in);
-            const DecItem b = P.items[i1];
-            if (pairable(a, b)) {
-                uint8_t *dst = reinterpret_cast<uint8_t *>(a.dst);
-                for (int r = tid; r < 256; r += 128) {
-                    const int z = r >> 4, y = r & 15;
-                    uint4 *row = reinterpret_cast<uint4 *>(dst + z * a.sz + y * a.sy);
-                    row[0] = *reinterpret_cast<const uint4 *>(sStage0 + z * kStageZ + y * 16);
-                    row[1] = *reinterpret_cast<const uint4 *>(sStage1 + z * kStageZ + y * 16);
-                }
-            } else {
-                store_block(a, sStage0);
-                store_block(b, sStage1);
-            }
-        } else {
-            store_block(a, sStage0);
+// One line-group step of the warp-wide passes: 4 adjacent lines x 2 outputs,
+// like lines4, with packed adds. A product must not reach a packed add inside
+// one basic block (see madd2), so the loop is software-pipelined: an iteration
+// adds the products of the previous one and computes its own, and the products
+// pass through the loop's back edge. #pragma unroll 1 keeps it so. K is even
+// and at least 4: a sum over fewer inputs takes zeros up to that, which add
+// +/-0, and starts from its first products (see lines4).
+__device__ __forceinline__ void mul_even(Acc4 &q, float4 v, float4 w) {
+    q.e0a = mul2(lo2(w), lo2(v)); q.e0b = mul2(lo2(w), hi2(v));
+    q.e1a = mul2(hi2(w), lo2(v)); q.e1b = mul2(hi2(w), hi2(v));
+}
+__device__ __forceinline__ void mul_odd(Acc4 &q, float4 v, float4 w) {
+    q.o0a = mul2(lo2(w), lo2(v)); q.o0b = mul2(lo2(w), hi2(v));
+    q.o1a = mul2(hi2(w), lo2(v)); q.o1b = mul2(hi2(w), hi2(v));
+}
+__device__ __forceinline__ void add_pending(Acc4 &a, const Acc4 &q) {
+    a.e0a = add2(a.e0a, q.e0a); a.e0b = add2(a.e0b, q.e0b);
+    a.e1a = add2(a.e1a, q.e1a); a.e1b = add2(a.e1b, q.e1b);
+    a.o0a = add2(a.o0a, q.o0a); a.o0b = add2(a.o0b, q.o0b);
+    a.o1a = add2(a.o1a, q.o1a); a.o1b = add2(a.o1b, q.o1b);
+}
+__device__ __forceinline__ Acc4 lines4p(const float4 *in, int ks, int K, const float4 *W) {
+    Acc4 a, q;
+    mul_even(a, in[0], W[0]);
+    mul_odd(a, in[ks], W[8]);
+    mul_even(q, in[2 * ks], W[16]);
+    mul_odd(q, in[3 * ks], W[24]);
+    if (K > 4) {
+        // inputs and weights are loaded an iteration ahead
+        float4 v = in[4 * ks], w = W[32], u = in[5 * ks], x = W[40];
+#pragma unroll 1
+        for (int k = 6;; k += 2) {
+            add_pending(a, q);
+            mul_even(q, v, w);
+            mul_odd(q, u, x);
+            if (k >= K) break;
+            in += 2 * ks;
+            W += 16;
+            v = in[4 * ks]; w = W[32]; u = in[5 * ks]; x = W[40];
         }
+    }
+    add_pending(a, q);
+    return a;
+}
+
+// Four voxels of a fast block: x, x + 1 | x + 2, x + 3 rounded by a packed magic add.
+__device__ __forceinline__ uint32_t pack4_fast2(float2 a, float2 b, int bias) {
+    const float2 mg = make_float2(12582912.0f, 12582912.0f);
+    const float2 fa = add2(a, mg), fb = add2(b, mg);
+    uint32_t t, d;
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, 0;" : "=r"(t) : "r"(__float_as_int(fb.y) + bias), "r"(__float_as_int(fb.x) + bias));
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(__float_as_int(fa.y) + bias), "r"(__float_as_int(fa.x) + bias), "r"(t));
+    return d;
+}
+
+// The same for voxels of any size (corrupt streams only).
+__device__ __noinline__ uint32_t pack4_slow(float2 a, float2 b, int dc) { return pack4(a, b, dc); }
+
+// Shared memory of k_reconstruct: the weights ([k][m/2], as c_cos2), the
+// coefficient box, whose planes become the pass-2 output in place (kBoxPlane
+// floats each), and for each of the two warps the pass-1 output of the planes it
+// works on, later the stage of its half of the rows (warp w: y >> 3 == w,
+// [z][y & 7][x]).
+struct RecSmem {
+    float4 W[16 * 8];
+    float box[kBoxB];
+    float a[2][32 * kRowF];
+    uint32_t ext[2];    // per warp: largest cz << 8 | cy << 4 | cx, each coordinate on its own
+    float l1[2];
+};
+constexpr int kStageHalf = sizeof(float) * 32 * kRowF;   // bytes from row 0's slice to row 8's
+__device__ __forceinline__ int stage_at(int z, int y) { return (y >> 3) * kStageHalf + z * 128 + (y & 7) * 16; }
+
+// Pass 3 of the warp's 32 line groups, outputs m = 4 half + j and 15 - m of 4
+// adjacent z-lines: in[k * kBoxPlane/4] the k-th inputs; the four voxels at z =
+// m to word j, at z = 15 - m to word 4 + j.
+struct Acc8 { float2 ea[4], eb[4], oa[4], ob[4]; };   // even and odd sums, lines 0-1 and 2-3
+__device__ __forceinline__ void mul8(float2 *a, float2 *b, float4 v, const float4 *w) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const float4 c = w[j];
+        a[2 * j] = mul2(lo2(c), lo2(v)); b[2 * j] = mul2(lo2(c), hi2(v));
+        a[2 * j + 1] = mul2(hi2(c), lo2(v)); b[2 * j + 1] = mul2(hi2(c), hi2(v));
+    }
+}
+__device__ __forceinline__ void add_pending8(Acc8 &a, const Acc8 &q) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        a.ea[j] = add2(a.ea[j], q.ea[j]); a.eb[j] = add2(a.eb[j], q.eb[j]);
+        a.oa[j] = add2(a.oa[j], q.oa[j]); a.ob[j] = add2(a.ob[j], q.ob[j]);
+    }
+}
+__device__ __forceinline__ void pass3(const float4 *in, int E, int half, int dc, bool fast, uint32_t word[8]) {
+    constexpr int ks = kBoxPlane / 4;
+    const float4 *w = c_cos2[0] + 2 * half;
+    Acc8 a, q;
+    mul8(a.ea, a.eb, in[0], w);
+    mul8(a.oa, a.ob, in[ks], w + 8);
+    mul8(q.ea, q.eb, in[2 * ks], w + 16);
+    mul8(q.oa, q.ob, in[3 * ks], w + 24);
+    if (E > 4) {
+        float4 v = in[4 * ks], u = in[5 * ks];   // loaded an iteration ahead
+#pragma unroll 1
+        for (int k = 6;; k += 2) {
+            add_pending8(a, q);
+            w += 16;
+            mul8(q.ea, q.eb, v, w + 16);
+            mul8(q.oa, q.ob, u, w + 24);
+            if (k >= E) break;
+            in += 2 * ks;
+            v = in[4 * ks];
+            u = in[5 * ks];
+        }
+    }
+    add_pending8(a, q);
+    const int bias = dc - 0x4B400000;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 p0 = add2(a.ea[j], a.oa[j]), p1 = add2(a.eb[j], a.ob[j]);
+        const float2 q0 = sub2(a.ea[j], a.oa[j]), q1 = sub2(a.eb[j], a.ob[j]);
+        word[j] = fast ? pack4_fast2(p0, p1, bias) : pack4_slow(p0, p1, dc);
+        word[4 + j] = fast ? pack4_fast2(q0, q1, bias) : pack4_slow(q0, q1, dc);
+    }
+}
+
+// The reconstruction stage of a batch: two warps per block. The first two
+// passes go a few planes at a time (as many as fill a warp's 32 lanes with pass-1
+// groups), plane groups in turn to the two warps, each through its own small
+// pass-1 buffer, and leave their output in the box's own planes. So a block
+// needs 25 KB of shared memory instead of the 43 KB of the CTA-wide routine
+// (reconstruct_block, for the kernels that decode few blocks or hold one CTA's
+// memory for both stages): nine blocks at a time on an SM instead of five, with
+// half the warps issuing the work outside the transforms (headers, entry
+// scatter, reductions, stores). The last pass gives a lane 8 of a line group's 16
+// outputs at a time and takes its weights from constant memory by a warp-uniform
+// index; all sums are packed adds (see lines4p).
+// What bounds it: latency, at 18 warps an SM and 0.43 instructions a cycle and
+// scheduler (3130 a block at q=6, 3960 before). 64 chunks at q=6 1.61 ms, at q=12
+// 1.16; with reconstruct_block on 4-warp CTAs 1.87 and 1.51. Tried and dropped:
+// one warp per block without barriers (10 warps an SM, 1.87), pairs of blocks
+// with 32-byte row stores (16 registers held over a block, spills: 1.70).
+__global__ void __launch_bounds__(64, 9) k_reconstruct(RecParams P) {
+    extern __shared__ __align__(16) uint8_t s_rec[];
+    RecSmem &S = *reinterpret_cast<RecSmem *>(s_rec);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < 16 * 8; i += 64) S.W[i] = c_cos2[i >> 3][i & 7];
+    for (int i = tid; i < kBoxB / 4; i += 64) reinterpret_cast<float4 *>(S.box)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    const int nb = gridDim.x;
+    const int mh = lane & 3, m = mh * 2;
+    float *const A = S.a[warp];
+    uint8_t *const stage = reinterpret_cast<uint8_t *>(S.a);
+    // the next block's header, entry offset and payload length, loaded while
+    // this one is transformed; then its first 256 entries, while pass 3 runs
+    int i = blockIdx.x;
+    EntHdr hn = {};
+    uint64_t basen = 0;
+    uint32_t lenn = 0, slotn = 0, en[4] = {0, 0, 0, 0};
+    auto next_head = [&](int j) {
+        const int item = P.idx ? (int)__ldg(P.idx + j) : j;
+        hn = load_hdr<false>(P.hdr + item);
+        basen = P.base[item];
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(&P.items[item].len));
+        lenn = v.x;
+        slotn = v.y & 0xFFFFu;
+    };
+    auto next_entries = [&]() {
+        const int lim = lenn && hn.nnz <= kN3 ? min((int)hn.nnz, (int)entry_cap(lenn)) : 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (tid + 64 * k < lim) en[k] = P.arena[basen + tid + 64 * k];
+    };
+    if (i < P.n) {
+        next_head(i);
+        next_entries();
+    }
+    for (; i < P.n; i += nb) {
+        const int item = P.idx ? (int)__ldg(P.idx + i) : i;
+        const DecItem it = P.items[item];
+        const EntHdr h = hn;
+        const uint64_t base = basen;
+        const uint32_t len = lenn, cap = entry_cap(lenn), nslot = slotn;
+        if (i + nb < P.n) next_head(i + nb);
+        // the header comes from k_entropy; the guards keep every index below
+        // inside shared memory whatever its contents
+        const bool sane = h.nnz <= kN3 && h.ncorr <= kN3;
+        const int dc = len && sane ? h.dc : 0;
+        const int nnz = len && sane ? h.nnz : 0;
+        const int ncorr = len && sane ? h.ncorr : 0;
+        int E = 0;   // box planes that this block wrote
+        if (nnz == 0) {
+            // constant block (src/mc_codec.c:757-759) or absent block (zeros)
+            const uint32_t w = (uint32_t)dc * 0x01010101u;
+            if (!ncorr && it.clip_lo == kClipFullLo && it.clip_hi == kClipFullHi) {
+                uint8_t *dst = reinterpret_cast<uint8_t *>(it.dst) + (tid & 15) * it.sy + (tid >> 4) * it.sz;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) store_row16(dst + 4 * j * it.sz, make_uint4(w, w, w, w));
+                if (i + nb < P.n) next_entries();
+                continue;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                reinterpret_cast<uint4 *>(stage + warp * kStageHalf)[j * 32 + lane] = make_uint4(w, w, w, w);
+            if (i + nb < P.n) next_entries();
+        } else {
+            // one pass over the entries, as in reconstruct_block
+            const QTab &qt = P.qtab[nslot];
+            int mz = 0, my = 0, mx = 0;
+            float l1 = 0.0f;
+            for (int j0 = tid; j0 < nnz; j0 += 256) {
+                uint32_t e[4], ix[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int j = j0 + 64 * k;
+                    e[k] = j < nnz ? (j0 < 64 && j < (int)cap ? en[k] : entry_at<false>(P, base, cap, h.ovf, j)) : 0u;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) ix[k] = j0 + 64 * k < nnz ? __ldg(P.scan + (e[k] & 0xFFFu)) & 0xFFFu : 0u;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (j0 + 64 * k >= nnz) break;
+                    const int idx = (int)ix[k];
+                    const int cz = idx >> 8, cy = (idx >> 4) & 15, cx = idx & 15;
+                    mz = max(mz, cz);
+                    my = max(my, cy);
+                    mx = max(mx, cx);
+                    const int lv = (int16_t)(e[k] >> 16);
+                    if (lv) {
+                        const int f = cz + cy + cx;
+                        const float a = (float)(lv < 0 ? -lv : lv);
+                        const float r = fadd(fadd(fmul(fsub(a, 1.0f), qt.step[f]), qt.dz8[f]), qt.dz4[f]);
+                        S.box[cz * kBoxPlane + cx * 16 + cy] = lv < 0 ? -r : r;
+                        l1 = fadd(l1, r);
+                    }
+                }
+            }
+            mz = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)mz);
+            my = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)my);
+            mx = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)mx);
+            for (int o = 16; o > 0; o >>= 1) l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, o);
+            if (lane == 0) {
+                S.ext[warp] = (uint32_t)(mz << 8 | my << 4 | mx);
+                S.l1[warp] = l1;
+            }
+            __syncthreads();   // the box is complete
+            const uint32_t x0 = S.ext[0], x1 = S.ext[1];
+            E = (int)max(x0 >> 8, x1 >> 8) + 1;
+            const int Y = (int)max((x0 >> 4) & 15u, (x1 >> 4) & 15u) + 1, X = (int)max(x0 & 15u, x1 & 15u) + 1;
+            const bool fast = S.l1[0] + S.l1[1] < kFastL1;
+            // even numbers of inputs, at least 4 (see lines4p)
+            const int Ee = max((E + 1) & ~1, 4), Ye = max((Y + 1) & ~1, 4), Xe = max((X + 1) & ~1, 4);
+            // passes 1 and 2 over np planes at a time: G groups of 4 lines a plane
+            const int G = (Y + 3) >> 2;
+            const int np = G == 1 ? 8 : (G == 2 ? 4 : 2);
+            const int gi = lane >> 2;
+            const int lp = G == 1 ? gi : (G == 2 ? gi >> 1 : (G == 3 ? (gi * 11) >> 5 : gi >> 2));   // gi / G
+            const int cy0 = (gi - lp * G) << 2;
+            for (int c0 = warp * np; c0 < E; c0 += 2 * np) {
+                if (lp < np && c0 + lp < E) {
+                    const Acc4 a = lines4p(reinterpret_cast<const float4 *>(S.box + (c0 + lp) * kBoxPlane + cy0), 4, Xe,
+                                           S.W + mh);
+                    // line i of the group: outputs m, m+1 (e + o) and 15-m, 14-m (e - o)
+                    const float2 p0 = add2(a.e0a, a.o0a), p1 = add2(a.e0b, a.o0b);
+                    const float2 q0 = add2(a.e1a, a.o1a), q1 = add2(a.e1b, a.o1b);
+                    const float2 r0 = sub2(a.e0a, a.o0a), r1 = sub2(a.e0b, a.o0b);
+                    const float2 s0 = sub2(a.e1a, a.o1a), s1 = sub2(a.e1b, a.o1b);
+                    float *out = A + (lp * (4 * G) + cy0) * kRowF;
+                    *reinterpret_cast<float2 *>(out + m) = make_float2(p0.x, q0.x);
+                    *reinterpret_cast<float2 *>(out + 14 - m) = make_float2(s0.x, r0.x);
+                    *reinterpret_cast<float2 *>(out + kRowF + m) = make_float2(p0.y, q0.y);
+                    *reinterpret_cast<float2 *>(out + kRowF + 14 - m) = make_float2(s0.y, r0.y);
+                    *reinterpret_cast<float2 *>(out + 2 * kRowF + m) = make_float2(p1.x, q1.x);
+                    *reinterpret_cast<float2 *>(out + 2 * kRowF + 14 - m) = make_float2(s1.x, r1.x);
+                    *reinterpret_cast<float2 *>(out + 3 * kRowF + m) = make_float2(p1.y, q1.y);
+                    *reinterpret_cast<float2 *>(out + 3 * kRowF + 14 - m) = make_float2(s1.y, r1.y);
+                }
+                __syncwarp();
+                // A[plane][k][x..x+3] -> box plane [y][x..x+3], float4 groups swizzled (see bswz)
+                const int npl = min(np, E - c0);
+                for (int t = lane; t < npl * 16; t += 32) {
+                    const int xg = (t >> 2) & 3, pl = t >> 4;
+                    const Acc4 a = lines4p(reinterpret_cast<const float4 *>(A + pl * (4 * G) * kRowF + xg * 4), kRowF / 4,
+                                           Ye, S.W + mh);
+                    float *ob = S.box + (c0 + pl) * kBoxPlane;
+                    const int ga = (xg ^ mh) << 2, gb = (xg ^ (3 - mh)) << 2;
+                    const float2 p0 = add2(a.e0a, a.o0a), p1 = add2(a.e0b, a.o0b);
+                    const float2 q0 = add2(a.e1a, a.o1a), q1 = add2(a.e1b, a.o1b);
+                    const float2 r0 = sub2(a.e0a, a.o0a), r1 = sub2(a.e0b, a.o0b);
+                    const float2 s0 = sub2(a.e1a, a.o1a), s1 = sub2(a.e1b, a.o1b);
+                    *reinterpret_cast<float4 *>(ob + m * kRowB + ga) = make_float4(p0.x, p0.y, p1.x, p1.y);
+                    *reinterpret_cast<float4 *>(ob + (m + 1) * kRowB + ga) = make_float4(q0.x, q0.y, q1.x, q1.y);
+                    *reinterpret_cast<float4 *>(ob + (15 - m) * kRowB + gb) = make_float4(r0.x, r0.y, r1.x, r1.y);
+                    *reinterpret_cast<float4 *>(ob + (14 - m) * kRowB + gb) = make_float4(s0.x, s0.y, s1.x, s1.y);
+                }
+                __syncwarp();
+            }
+            if (i + nb < P.n) next_entries();
+            __syncthreads();   // every plane has its pass-2 output
+            // pass 3: lane l of warp w takes the group (y, xg) = (8 w + (l >> 2), l & 3)
+            const int y = 8 * warp + (lane >> 2);
+            const float4 *in = reinterpret_cast<const float4 *>(S.box + y * kRowB + (((lane & 3) ^ bswz(y)) << 2));
+            uint32_t *out = reinterpret_cast<uint32_t *>(A) + lane;   // the pass-1 buffer is free
+#pragma unroll 1
+            for (int half = 0; half < 2; ++half) {
+                uint32_t word[8];
+                pass3(in, Ee, half, dc, fast, word);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    out[(4 * half + j) * 32] = word[j];
+                    out[(15 - 4 * half - j) * 32] = word[4 + j];
+                }
+            }
+        }
+        if (ncorr) {
+            __syncthreads();
+            if (tid == 0) {
+                // corrections in stream order: a position may repeat, each
+                // application clamps (src/mc_codec.c:775-781)
+                for (int c = 0; c < ncorr; ++c) {
+                    const uint32_t pos = entry_at<false>(P, base, cap, h.ovf, nnz + 2 * c);
+                    const uint32_t d = entry_at<false>(P, base, cap, h.ovf, nnz + 2 * c + 1);
+                    if (pos >= (uint32_t)kN3) break;
+                    uint8_t &vox = stage[stage_at(pos >> 8, (pos >> 4) & 15) + (pos & 15)];
+                    const int v = (int)((uint32_t)vox + d);
+                    vox = (uint8_t)(v < 0 ? 0 : v > 255 ? 255 : v);
+                }
+            }
+            __syncthreads();
+        }
+        __syncwarp();
+        if (it.clip_lo == kClipFullLo && it.clip_hi == kClipFullHi) {
+            // each warp the rows it staged
+            uint8_t *dst = reinterpret_cast<uint8_t *>(it.dst) + (8 * warp + (lane & 7)) * it.sy + (lane >> 3) * it.sz;
+            const uint4 *row = reinterpret_cast<const uint4 *>(stage + warp * kStageHalf) + lane;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) store_row16(dst + 4 * j * it.sz, row[32 * j]);
+            __syncthreads();   // the box is read
+        } else {
+            __syncthreads();
+            store_block(it, [&](int z, int yy) { return stage + stage_at(z, yy); }, tid, 64);
+        }
+        for (int j = tid; j < E * (kBoxPlane / 4); j += 64)
+            reinterpret_cast<float4 *>(S.box)[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         __syncthreads();
     }
 }
@@ -1310,11 +1626,11 @@ __device__ __forceinline__ void reconstruct_pair(const RecParams &P, int j, floa
                 row[1] = *reinterpret_cast<const uint4 *>(stage1 + z * kStageZ + y * 16);
             }
         } else {
-            store_block(a, stage0);
-            store_block(b, stage1);
+            store_block(a, StageRows{stage0}, tid, 128);
+            store_block(b, StageRows{stage1}, tid, 128);
         }
     } else {
-        store_block(a, stage0);
+        store_block(a, StageRows{stage0}, tid, 128);
     }
 }
 
@@ -1487,7 +1803,7 @@ __global__ void __launch_bounds__(128) k_decode_one(DecItem it, SoloScratch *S, 
     R.qtab = qtab;
     R.scan = scan;
     reconstruct_block<true>(R, 0, sA, sB, sStage, sW);   // written in this kernel: read through L2
-    store_block(it, sStage);
+    store_block(it, StageRows{sStage}, tid, 128);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -1514,7 +1830,11 @@ cudaError_t upload_decode_tables(const float cmf[16][16], const uint16_t scan[kN
     }
     bend[7] = kN3;
     bend[8] = 0xFFFF;
-    const cudaError_t e = cudaMemcpyToSymbolAsync(c_cos, cmf, sizeof(float) * 256, 0, cudaMemcpyHostToDevice, s);
+    static float pairs[16][16][2];
+    for (int k = 0; k < 16; ++k)
+        for (int m = 0; m < 16; ++m) pairs[k][m][0] = pairs[k][m][1] = cmf[k][m];
+    cudaError_t e = cudaMemcpyToSymbolAsync(c_cos, cmf, sizeof(float) * 256, 0, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(c_cos2, pairs, sizeof pairs, 0, cudaMemcpyHostToDevice, s);
     return e != cudaSuccess ? e : cudaMemcpyToSymbolAsync(c_bend, bend, sizeof bend, 0, cudaMemcpyHostToDevice, s);
 }
 
@@ -1610,17 +1930,20 @@ cudaError_t launch_fused(const FusedParams &f, const LaunchCfg &cfg, cudaStream_
 
 cudaError_t launch_reconstruct(const RecParams &p, const LaunchCfg &cfg, cudaStream_t s) {
     if (p.n <= 0) return cudaSuccess;
-    int blocks = (p.n + 1) / 2;   // one CTA step per pair of blocks
-    int cap = num_sms() * (cfg.rec_ctas_per_sm > 0 ? cfg.rec_ctas_per_sm : 5);
-    if (blocks > cap) blocks = cap;
-    // per device: the largest shared-memory carveout, so that 5 CTAs per SM fit
-    static std::atomic<int> carve_set[kMaxDevs];
-    dev_once(carve_set, [] {
-        cudaFuncSetAttribute(k_reconstruct, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-        return 1;
+    // the knob counts 128 threads per SM as one: two CTAs of 64, of which 9 fit
+    const int per_sm = std::min(2 * (cfg.rec_ctas_per_sm > 0 ? cfg.rec_ctas_per_sm : 5), 9);
+    const int blocks = std::min(p.n, num_sms() * per_sm);
+    // per device: the dynamic shared memory opt-in and the largest carveout, so that 9 CTAs per SM fit
+    static std::atomic<int> attr[kMaxDevs];
+    const int a = dev_once(attr, [] {
+        cudaError_t e = cudaFuncSetAttribute(k_reconstruct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RecSmem));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_reconstruct, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     (int)cudaSharedmemCarveoutMaxShared);
+        return e == cudaSuccess ? 1 : -(int)e;
     });
-    k_reconstruct<<<blocks, 128, 0, s>>>(p);
+    if (a < 0) return (cudaError_t)(-a);
+    k_reconstruct<<<blocks, 64, sizeof(RecSmem), s>>>(p);
     return cudaGetLastError();
 }
 

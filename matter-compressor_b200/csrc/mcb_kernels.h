@@ -12,7 +12,7 @@ struct LaunchCfg {
     int ent_warps = 4;         // entropy stage: warps per CTA (2, 4 or 8)
     int ent_claim = 1;         // entropy stage: queue entries a lane claims at a time (1, 2 or 4)
     int ent_ctas_per_sm = 5;   // entropy stage: CTAs per SM (8.8 KB of contexts per warp)
-    int rec_ctas_per_sm = 4;   // reconstruction stage: CTAs of 128 threads per SM (<= 4: 47 KB smem)
+    int rec_ctas_per_sm = 5;   // reconstruction stage: 128 threads (two CTAs) per SM each; 5 is the most that fits
     int ent_solo = -1;         // entropy stage: the longest ncoded / ent_solo blocks are decoded one per
                                // warp by a single thread (0: none; see EntParams::nsolo); 1: every
                                // block, by the single-thread kernel k_entropy_solo; -1: by the
