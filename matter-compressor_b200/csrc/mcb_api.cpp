@@ -923,16 +923,28 @@ int mc_b200_append_chunks(mc_archive *a, mc_codec_ctx *C, int lod, const int *co
         if (!encode_chunks(*L, dv.data(), g, hq.data(), qq.data(), tau.data(), boff, blen)) return -1;
         uint64_t total = 0;
         for (int j = 0; j < g; ++j) total = std::max(total, boff[j] + blen[j]);
-        if (!L->h_stage.ensure(total + 16)) return -1;
-        if (total && !cuda_ok(cudaMemcpy(L->h_stage.p, L->blobs.p, total, cudaMemcpyDeviceToHost), "D2H blobs"))
+        if (!L->h_stage.ensure(total + 16)) {
+            encode_hashes(*L, g);
             return -1;
-        for (int j = 0; j < g; ++j) {
-            const int *cc = coords + 3 * (c0 + j);
-            int rc;
-            if (blen[j]) rc = install_blob(a, lod, cc[0], cc[1], cc[2], L->h_stage.as<uint8_t>() + boff[j], blen[j]);
-            else rc = C ? mark_zero(a, lod, cc[0], cc[1], cc[2]) : 0;   // all air
-            if (rc) return rc;
         }
+        // the blobs are copied out and written to the file while their hashes
+        // are computed; then each is published, in call order
+        bool ok = !total || (cuda_ok(cudaMemcpyAsync(L->h_stage.p, L->blobs.p, total, cudaMemcpyDeviceToHost,
+                                                     L->stream), "D2H blobs") &&
+                             finish(*L, nullptr));
+        PlacedBlob placed[G];
+        int rc = 0, np = 0;
+        for (; ok && np < g; ++np) {
+            const int *cc = coords + 3 * (c0 + np);
+            if (!blen[np] && !C) continue;   // the parallel path leaves all-air chunks out
+            rc = place_blob(a, lod, cc[0], cc[1], cc[2], L->h_stage.as<uint8_t>() + boff[np], blen[np], &placed[np]);
+            if (rc) break;
+        }
+        const uint64_t *hash = encode_hashes(*L, g);
+        if (!ok || !hash) return -1;
+        for (int j = 0; j < np; ++j)
+            if (blen[j] || C) commit_blob(a, placed[j], hash[j]);
+        if (rc) return rc;
     }
     return 0;
 }

@@ -146,16 +146,6 @@ uint64_t ensure_shard_slot(mc_archive *a, int lod, int cz, int cy, int cx) {
 }  // namespace
 
 namespace mcb {
-// src/mc_archive.c:447-456
-int mark_zero(mc_archive *a, int lod, int cz, int cy, int cx) {
-    std::lock_guard<std::mutex> g(a->write_mu);
-    uint64_t slot = ensure_shard_slot(a, lod, cz, cy, cx);
-    if (slot == ~0ull) return -1;
-    wr64(a->base + slot, kSlotZero);
-    touch(a, slot, 8);
-    a->gen.fetch_add(1, std::memory_order_release);
-    return 0;
-}
 // Bytes into the file at off, seen through the shared mapping at once (one
 // page cache): pwrite fills the pages without a fault per page of the
 // mapping, which a memcpy into freshly allocated file pages takes.
@@ -170,20 +160,47 @@ static void write_file(mc_archive *a, uint64_t off, const uint8_t *src, size_t l
     if (done < len) memcpy(a->base + off + done, src + done, len - done);
 }
 
-// src/mc_archive.c:458-485
-int install_blob(mc_archive *a, int lod, int cz, int cy, int cx, const uint8_t *blob, size_t len) {
-    std::lock_guard<std::mutex> g(a->write_mu);
-    uint64_t slot = ensure_shard_slot(a, lod, cz, cy, cx);
-    if (slot == ~0ull) return -1;
-    uint64_t off = alloc_at_eof(a, len);
-    if (off == ~0ull) return -1;
-    write_file(a, off, blob, len);
-    slot_at(a, slot)->store(off, std::memory_order_release);
+// Stores what a slot points to and, for a blob, the archive's length.
+static void publish_slot(mc_archive *a, uint64_t slot, uint64_t value) {
+    slot_at(a, slot)->store(value, std::memory_order_release);
     touch(a, slot, 8);
     a->gen.fetch_add(1, std::memory_order_release);
+    if (value == kSlotZero) return;
     uint64_t cur = a->cursor.load(std::memory_order_relaxed);
     slot_at(a, HTOTLEN)->store(cur, std::memory_order_relaxed);
     touch(a, HTOTLEN, 8);
+}
+
+// src/mc_archive.c:458-485, and :447-456 for an all-air chunk
+int place_blob(mc_archive *a, int lod, int cz, int cy, int cx, const uint8_t *blob, size_t len, PlacedBlob *out) {
+    std::lock_guard<std::mutex> g(a->write_mu);
+    out->slot = ensure_shard_slot(a, lod, cz, cy, cx);
+    if (out->slot == ~0ull) return -1;
+    out->off = 0;
+    if (!len) return 0;
+    const uint64_t off = alloc_at_eof(a, len);
+    if (off == ~0ull) return -1;
+    write_file(a, off, blob, len);
+    out->off = off;
+    return 0;
+}
+
+void commit_blob(mc_archive *a, const PlacedBlob &b, uint64_t hash) {
+    std::lock_guard<std::mutex> g(a->write_mu);
+    if (!b.off) {
+        publish_slot(a, b.slot, kSlotZero);
+        return;
+    }
+    write_file(a, b.off + 4, reinterpret_cast<const uint8_t *>(&hash), 8);   // [f32 q][u64 hash]
+    touch(a, b.off + 4, 8);   // the mirror may have taken the blob in between
+    publish_slot(a, b.slot, b.off);
+}
+
+int install_blob(mc_archive *a, int lod, int cz, int cy, int cx, const uint8_t *blob, size_t len) {
+    PlacedBlob b;
+    if (place_blob(a, lod, cz, cy, cx, blob, len, &b) != 0) return -1;
+    std::lock_guard<std::mutex> g(a->write_mu);
+    publish_slot(a, b.slot, b.off);
     return 0;
 }
 
@@ -458,6 +475,7 @@ int mc_enc_block(mc_codec_ctx *C, const mc_u8 *vox, mc_buf *out, uint32_t *len_o
         !cuda_ok(cudaMemcpyAsync(L->enc_items.p, hs + kN3, sizeof it, cudaMemcpyHostToDevice, L->stream), "H2D") ||
         !cuda_ok(cudaMemsetAsync(L->status.p, 0, 16, L->stream), "memset") ||
         !cuda_ok(launch_encode(ep, L->stream), "encode launch") ||
+        !cuda_ok(launch_encode_rc(ep, L->stream), "range coder launch") ||
         !cuda_ok(cudaMemcpyAsync(&len, L->enc_len.p, 4, cudaMemcpyDeviceToHost, L->stream), "D2H") ||
         !cuda_ok(cudaStreamSynchronize(L->stream), "sync"))
         return 0;

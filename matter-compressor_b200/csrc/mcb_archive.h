@@ -49,7 +49,16 @@ struct ChunkIndex {
 const ChunkIndex &chunk_index(const uint8_t *arc, uint64_t chunk_off);
 float chunk_q(const mc_archive *a, uint64_t chunk_off);
 int install_blob(mc_archive *a, int lod, int cz, int cy, int cx, const uint8_t *blob, size_t len);
-int mark_zero(mc_archive *a, int lod, int cz, int cy, int cx);
+// The same in two steps, for a blob whose hash is not known yet: place_blob
+// reserves index slot and file range and writes the blob (len 0: the slot alone,
+// for an all-air chunk), commit_blob stores the hash in its header and publishes
+// it (or the all-air mark). A blob that is never committed is bytes that nothing
+// refers to.
+struct PlacedBlob {
+    uint64_t slot = 0, off = 0;   // off 0: all air
+};
+int place_blob(mc_archive *a, int lod, int cz, int cy, int cx, const uint8_t *blob, size_t len, PlacedBlob *out);
+void commit_blob(mc_archive *a, const PlacedBlob &b, uint64_t hash);
 // Bring the HBM mirror up to date and order the lane's stream after it.
 uint8_t *mirror_sync(mc_archive *a, Lane &L);
 // A chunk blob that passed the structural checks of the verify walk.

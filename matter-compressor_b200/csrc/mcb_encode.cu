@@ -8,7 +8,7 @@
 //   transform, lrint + dc, list every voxel whose error exceeds tau
 //   (:697-708) -> range coding of header bins, coefficients and corrections
 //   by one thread (the coder is a serial chain; src/mc_codec.c:178-233).
-// k_blob_layout / k_blob_fill / k_blob_hash: per-chunk blob assembly
+// k_fracmap / k_blob_layout / k_blob_fill / k_blob_hash: per-chunk blob assembly
 //   (src/mc_codec.c:809-845, src/mc_archive.c:861-901): bitmap + u16 lengths
 //   in block order, fraction map range-coded (src/mc_codec.c:600-611),
 //   payloads concatenated in block order, xxh64 chain over
@@ -375,10 +375,85 @@ __global__ void __launch_bounds__(128) k_encode_rc(EncParams P) {
 }
 
 // ------------------------------------------------------------ blob assembly
+// Fraction map of a chunk, range-coded by one thread (src/mc_codec.c:600-611):
+// a chain of 16384 bins, which needs only the transform's material nibbles, so
+// it runs on a stream of its own beside the block coder. Most nibbles repeat
+// one of the two extremes, air behind air (four 0 bins) or full behind full
+// (four 1 bins); such a nibble is coded straight through, the four splits
+// computed one from the other, when the last range shows that none of them
+// renormalises. One chunk or many: 0.95 ms as the tail of the sizing pass with
+// contexts in local memory, 0.75 ms here, beside the coder.
+__device__ __forceinline__ uint32_t up0(uint32_t p) { return p + ((4096u - p) >> 4); }
+__device__ __forceinline__ uint32_t up1(uint32_t p) { return p - (p >> 4); }
+__device__ __forceinline__ void frac_bit(Enc &e, uint32_t &p0, uint32_t bit) {
+    const uint32_t r0 = (e.range >> 12) * p0;
+    if (!bit) { e.range = r0; p0 = up0(p0); }
+    else { e.low += r0; e.range -= r0; p0 = up1(p0); }
+    enc_norm(e);
+}
+__device__ __forceinline__ void frac_nibble(Enc &e, uint32_t (&p)[4], uint32_t v) {
+    frac_bit(e, p[3], (v >> 3) & 1);
+    frac_bit(e, p[2], (v >> 2) & 1);
+    frac_bit(e, p[1], (v >> 1) & 1);
+    frac_bit(e, p[0], v & 1);
+}
+__global__ void __launch_bounds__(32) k_fracmap(BlobParams P) {
+    if (threadIdx.x) return;
+    const int c = blockIdx.x;
+    Enc e;
+    e.out = P.fmap + (size_t)c * kFmapCap;
+    e.cap = kFmapCap; e.len = 0; e.low = 0; e.range = 0xFFFFFFFFu; e.cache = 0; e.pending = 1;
+    uint32_t lo[4], mid[4], hi[4];   // contexts behind a nibble of 0, of 1..14, of 15
+#pragma unroll
+    for (int j = 0; j < 4; ++j) lo[j] = mid[j] = hi[j] = 2048;
+    const uint4 *fr = reinterpret_cast<const uint4 *>(P.frac + (size_t)c * kGrid3);
+    uint32_t prev = 0;
+    uint4 ahead = fr[0];
+    for (int i = 0; i < kGrid3 / 16; ++i) {
+        const uint4 now = ahead;
+        if (i + 1 < kGrid3 / 16) ahead = fr[i + 1];
+        const uint32_t w[4] = {now.x, now.y, now.z, now.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            uint32_t word = w[q];
+#pragma unroll 1
+            for (int b = 0; b < 4; ++b, word >>= 8) {
+                const uint32_t v = word & 15u;
+                if (prev == 0) {
+                    const uint32_t r1 = (e.range >> 12) * lo[3], r2 = (r1 >> 12) * lo[2];
+                    const uint32_t r3 = (r2 >> 12) * lo[1], r4 = (r3 >> 12) * lo[0];
+                    if (v == 0 && r4 >= (1u << 24)) {
+                        e.range = r4;
+                        lo[3] = up0(lo[3]); lo[2] = up0(lo[2]); lo[1] = up0(lo[1]); lo[0] = up0(lo[0]);
+                    } else {
+                        frac_nibble(e, lo, v);
+                    }
+                } else if (prev == 15) {
+                    const uint32_t s1 = (e.range >> 12) * hi[3], r1 = e.range - s1;
+                    const uint32_t s2 = (r1 >> 12) * hi[2], r2 = r1 - s2;
+                    const uint32_t s3 = (r2 >> 12) * hi[1], r3 = r2 - s3;
+                    const uint32_t s4 = (r3 >> 12) * hi[0], r4 = r3 - s4;
+                    if (v == 15 && r4 >= (1u << 24)) {
+                        e.low += (uint64_t)s1 + s2 + s3 + s4;
+                        e.range = r4;
+                        hi[3] = up1(hi[3]); hi[2] = up1(hi[2]); hi[1] = up1(hi[1]); hi[0] = up1(hi[0]);
+                    } else {
+                        frac_nibble(e, hi, v);
+                    }
+                } else {
+                    frac_nibble(e, mid, v);
+                }
+                prev = v;
+            }
+        }
+    }
+    for (int i = 0; i < 5; ++i) enc_shift(e);
+    P.fml[c] = e.len > (uint32_t)kFmapCap ? (uint32_t)kFmapCap : e.len;
+}
+
 // Sizing pass, one CTA of 1024 threads per chunk: block-order exclusive scans
-// of (present, bytes), the u16 length table and bitmap into side buffers, the
-// fraction map range-coded by one thread (src/mc_codec.c:600-611), and the
-// blob's total length (0 when every block is air).
+// of (present, bytes), the u16 length table and bitmap into side buffers, and
+// the blob's total length (0 when every block is air). After k_fracmap.
 __global__ void __launch_bounds__(1024) k_blob_layout(BlobParams P) {
     __shared__ uint32_t s_wnp[32], s_wby[32];
     const int c = blockIdx.x, tid = threadIdx.x;
@@ -421,27 +496,12 @@ __global__ void __launch_bounds__(1024) k_blob_layout(BlobParams P) {
         P.bitmap[(size_t)c * kBitmapBytes + tid] = (uint8_t)byte;
     }
     if (tid == 0) {
-        Enc e;
-        e.out = P.fmap + (size_t)c * kFmapCap;
-        e.cap = kFmapCap; e.len = 0; e.low = 0; e.range = 0xFFFFFFFFu; e.cache = 0; e.pending = 1;
-        uint16_t cx[3][4];
-        for (int i = 0; i < 3; ++i) for (int j = 0; j < 4; ++j) cx[i][j] = 2048;
-        const uint8_t *fr = P.frac + (size_t)c * kGrid3;
-        int prev = 0;
-        for (int i = 0; i < kGrid3; ++i) {
-            int v = fr[i] & 15, b = prev == 0 ? 0 : prev == 15 ? 2 : 1;
-            for (int bit = 3; bit >= 0; --bit) enc_bit(e, cx[b][bit], (v >> bit) & 1);
-            prev = v;
-        }
-        for (int i = 0; i < 5; ++i) enc_shift(e);
-        const uint32_t fml = e.len > (uint32_t)kFmapCap ? (uint32_t)kFmapCap : e.len;
-        P.fml[c] = fml;
         P.np[c] = np_total;
-        P.blob_len[c] = np_total ? (uint64_t)kBlobHdr + fml + kBitmapBytes + 2ull * np_total + by_total : 0;
+        P.blob_len[c] = np_total ? (uint64_t)kBlobHdr + P.fml[c] + kBitmapBytes + 2ull * np_total + by_total : 0;
     }
 }
 
-// Write pass: header (hash patched by k_blob_hash), fmap, bitmap, lengths and
+// Write pass: header (the hash is k_blob_hash's, patched into the installed blob), fmap, bitmap, lengths and
 // the payloads in block order. Grid (64, nchunks), a warp per block.
 __global__ void __launch_bounds__(256) k_blob_fill(BlobParams P) {
     const int c = blockIdx.y;
@@ -496,151 +556,142 @@ __device__ __forceinline__ uint64_t ld64u(const uint8_t *p) {
 
 }  // namespace
 
-// Device verify (src/mc_archive.c:1072-1111): the chained hash of every
-// listed blob of an archive held in device memory, compared with the hash
-// stored in the blob's header; bad[i] = 1 on a mismatch.
+// The chained hash of a blob (src/mc_archive.c:76-88), one CTA per blob.
 //
-// One warp per blob. XXH64 keeps 4 serial accumulators, so 4 lanes hash; the
-// whole warp first brings each 4 KiB tile of the blob into shared memory with
-// coalesced 16-byte loads (many in flight at once), and the hashing lanes then
-// read their stripes from shared memory: the serial round chain no longer
-// waits on memory for every stripe.
+// XXH64 keeps 4 serial accumulators, acc = rotl(acc + word * P2, 31) * P1, so
+// four lanes of the first warp hash and the other warps feed them: they read
+// the next tile's words (any alignment), multiply them by P2, which is off the
+// chain, and leave the products in shared memory while the current tile is
+// hashed. What is left on the chain is an add, a rotate and one multiply, and
+// nothing waits on memory. A blob of 6.3 MB: 10.05 ms with one warp loading and
+// hashing by turns, 4.2 ms so.
 namespace {
-constexpr int kVerifyWarps = 4;
+constexpr int kHashThreads = 128;
 constexpr int kTileStripes = 128;
-constexpr int kTileBytes = kTileStripes * 32;
-constexpr int kTileBuf = kTileBytes + 64;   // a window plus its misaligned head and tail
-
-// Bytes [start, start + n) of the archive into tile (n <= kTileBytes + 32),
-// from the 16-byte boundary at or below start; bytes outside [base, limit)
-// read 0. Returns that boundary. Every lane of the warp calls it.
-__device__ const uint8_t *load_window(const uint8_t *base, const uint8_t *limit, const uint8_t *start, uint32_t n,
-                                      uint8_t *tile) {
-    const int lane = threadIdx.x & 31;
-    const uint8_t *wb = reinterpret_cast<const uint8_t *>((uintptr_t)start & ~(uintptr_t)15);
-    const uint32_t nvec = (uint32_t)((start + n - wb + 15) / 16);
-    for (uint32_t i = lane; i < nvec; i += 32) {
-        const uint8_t *q = wb + 16 * i;
-        uint4 v;
-        if (q >= base && q + 16 <= limit) {
-            v = __ldg(reinterpret_cast<const uint4 *>(q));
-        } else {
-            uint8_t b[16];
-            for (int k = 0; k < 16; ++k) b[k] = (q + k >= base && q + k < limit) ? q[k] : 0;
-            memcpy(&v, b, 16);
-        }
-        reinterpret_cast<uint4 *>(tile)[i] = v;
-    }
-    __syncwarp();
-    return wb;
-}
-
-// 8 little-endian bytes at tile offset o (any alignment)
-__device__ __forceinline__ uint64_t tile64(const uint8_t *tile, uint32_t o) {
-    const uint32_t a = o & 7;
-    const uint64_t lo = *reinterpret_cast<const uint64_t *>(tile + (o - a));
-    if (!a) return lo;
-    const uint64_t hi = *reinterpret_cast<const uint64_t *>(tile + (o - a) + 8);
-    return (lo >> (8 * a)) | (hi << (64 - 8 * a));
-}
-
-// XXH64 of [p, p + len) by a whole warp through tile; the hash in every lane.
-__device__ uint64_t xxh64_warp(const uint8_t *base, const uint8_t *limit, const uint8_t *p, uint64_t len,
-                               uint64_t seed, uint8_t *tile) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t nstripes = len >= 32 ? len / 32 : 0;
-    uint64_t acc = lane == 0 ? seed + XP1 + XP2 : lane == 1 ? seed + XP2 : lane == 2 ? seed : seed - XP1;
-    for (uint64_t s0 = 0; s0 < nstripes; s0 += kTileStripes) {
-        const uint32_t n = (uint32_t)min((uint64_t)kTileStripes, nstripes - s0);
-        const uint8_t *start = p + 32 * s0;
-        const uint8_t *wb = load_window(base, limit, start, 32 * n, tile);
-        if (lane < 4) {
-            const uint32_t o0 = (uint32_t)(start - wb) + 8 * lane;
-#pragma unroll 8
-            for (uint32_t s = 0; s < n; ++s) acc = xround(acc, tile64(tile, o0 + 32 * s));
-        }
-        __syncwarp();
-    }
-    const uint64_t a0 = __shfl_sync(0xFFFFFFFFu, acc, 0), a1 = __shfl_sync(0xFFFFFFFFu, acc, 1);
-    const uint64_t a2 = __shfl_sync(0xFFFFFFFFu, acc, 2), a3 = __shfl_sync(0xFFFFFFFFu, acc, 3);
+struct HashSmem {
+    uint64_t prod[2][kTileStripes * 4];
     uint64_t h;
-    if (nstripes) {
-        h = rotl64(a0, 1) + rotl64(a1, 7) + rotl64(a2, 12) + rotl64(a3, 18);
-        h = (h ^ xround(0, a0)) * XP1 + XP4;
-        h = (h ^ xround(0, a1)) * XP1 + XP4;
-        h = (h ^ xround(0, a2)) * XP1 + XP4;
-        h = (h ^ xround(0, a3)) * XP1 + XP4;
-    } else {
-        h = seed + XP5;
+};
+
+// 8 little-endian bytes at q; aligned loads inside [base, limit), bytes
+// outside it read 0.
+__device__ __forceinline__ uint64_t word64(const uint8_t *base, const uint8_t *limit, const uint8_t *q) {
+    const uint32_t a = (uint32_t)(uintptr_t)q & 7u;
+    const uint8_t *w = q - a;
+    if (w >= base && w + 16 <= limit) {
+        const uint64_t lo = __ldg(reinterpret_cast<const unsigned long long *>(w));
+        if (!a) return lo;
+        const uint64_t hi = __ldg(reinterpret_cast<const unsigned long long *>(w) + 1);
+        return (lo >> (8 * a)) | (hi << (64 - 8 * a));
     }
-    h += len;
-    // the tail (< 32 bytes) by every lane alike, from one more window
-    const uint8_t *t = p + nstripes * 32;
-    const uint32_t rem = (uint32_t)(len - nstripes * 32);
-    const uint8_t *wb = load_window(base, limit, t, rem, tile);
-    uint32_t o = (uint32_t)(t - wb), end = o + rem;
-    for (; end - o >= 8; o += 8) h = rotl64(h ^ xround(0, tile64(tile, o)), 27) * XP1 + XP4;
-    if (end - o >= 4) {
-        const uint64_t w = tile64(tile, o) & 0xFFFFFFFFull;
-        h = rotl64(h ^ (w * XP1), 23) * XP2 + XP3;
-        o += 4;
+    uint64_t v = 0;
+    for (int k = 7; k >= 0; --k) v = (v << 8) | (q + k >= base && q + k < limit ? q[k] : 0);
+    return v;
+}
+
+// XXH64 of [p, p + len) by the whole CTA; the hash in every thread.
+__device__ uint64_t xxh64_cta(const uint8_t *base, const uint8_t *limit, const uint8_t *p, uint64_t len, uint64_t seed,
+                              HashSmem &S) {
+    const int tid = threadIdx.x;
+    const uint64_t nstripes = len / 32;
+    const uint64_t ntiles = (nstripes + kTileStripes - 1) / kTileStripes;
+    auto stripes_of = [&](uint64_t t) { return (int)min((uint64_t)kTileStripes, nstripes - t * kTileStripes); };
+    auto fill = [&](uint64_t t, int first, int step) {
+        const uint8_t *q = p + t * (kTileStripes * 32);
+        const int n = stripes_of(t) * 4;
+        for (int w = first; w < n; w += step) S.prod[t & 1][w] = word64(base, limit, q + 8 * w) * XP2;
+    };
+    uint64_t acc = tid == 0 ? seed + XP1 + XP2 : tid == 1 ? seed + XP2 : tid == 2 ? seed : seed - XP1;
+    if (ntiles) fill(0, tid, kHashThreads);
+    __syncthreads();
+    for (uint64_t t = 0; t < ntiles; ++t) {
+        if (tid < 4) {
+            const uint64_t *pr = S.prod[t & 1] + tid;
+            const int n = stripes_of(t);
+#pragma unroll 8
+            for (int s = 0; s < n; ++s) acc = rotl64(acc + pr[4 * s], 31) * XP1;
+        } else if (tid >= 32 && t + 1 < ntiles) {
+            fill(t + 1, tid - 32, kHashThreads - 32);
+        }
+        __syncthreads();
     }
-    for (; o < end; ++o) h = rotl64(h ^ ((uint64_t)tile[o] * XP5), 11) * XP1;
-    h ^= h >> 33; h *= XP2; h ^= h >> 29; h *= XP3; h ^= h >> 32;
-    __syncwarp();   // the tile is reused by the next call
+    if (tid < 32) {
+        const uint64_t a0 = __shfl_sync(0xFFFFFFFFu, acc, 0), a1 = __shfl_sync(0xFFFFFFFFu, acc, 1);
+        const uint64_t a2 = __shfl_sync(0xFFFFFFFFu, acc, 2), a3 = __shfl_sync(0xFFFFFFFFu, acc, 3);
+        if (tid == 0) {
+            uint64_t h;
+            if (nstripes) {
+                h = rotl64(a0, 1) + rotl64(a1, 7) + rotl64(a2, 12) + rotl64(a3, 18);
+                h = (h ^ xround(0, a0)) * XP1 + XP4;
+                h = (h ^ xround(0, a1)) * XP1 + XP4;
+                h = (h ^ xround(0, a2)) * XP1 + XP4;
+                h = (h ^ xround(0, a3)) * XP1 + XP4;
+            } else {
+                h = seed + XP5;
+            }
+            h += len;
+            const uint8_t *q = p + nstripes * 32, *end = p + len;
+            for (; end - q >= 8; q += 8) h = rotl64(h ^ xround(0, word64(base, limit, q)), 27) * XP1 + XP4;
+            if (end - q >= 4) {
+                const uint64_t w = word64(base, limit, q) & 0xFFFFFFFFull;
+                h = rotl64(h ^ (w * XP1), 23) * XP2 + XP3;
+                q += 4;
+            }
+            for (; q < end; ++q) h = rotl64(h ^ ((word64(base, limit, q) & 0xFFull) * XP5), 11) * XP1;
+            h ^= h >> 33; h *= XP2; h ^= h >> 29; h *= XP3; h ^= h >> 32;
+            S.h = h;
+        }
+    }
+    __syncthreads();
+    const uint64_t h = S.h;
+    __syncthreads();   // S is reused by the next call
+    return h;
+}
+
+// Over fmap | bitmap | lengths | payloads of the blob at `blob`, len bytes, np
+// present blocks.
+__device__ uint64_t blob_hash_cta(const uint8_t *base, const uint8_t *limit, const uint8_t *blob, uint64_t len,
+                                  uint32_t np, HashSmem &S) {
+    const uint16_t fml = (uint16_t)(blob[12] | (blob[13] << 8));
+    const uint8_t *fmap = blob + kBlobHdr, *bm = fmap + fml, *lens = bm + kBitmapBytes;
+    const uint64_t pay = (uint64_t)kBlobHdr + fml + kBitmapBytes + 2ull * np;
+    uint64_t h = xxh64_cta(base, limit, fmap, fml, kHashSeed, S);
+    h ^= xxh64_cta(base, limit, bm, kBitmapBytes, h, S);
+    h ^= xxh64_cta(base, limit, lens, 2ull * np, h, S);
+    h ^= xxh64_cta(base, limit, blob + pay, len - pay, h, S);
     return h;
 }
 }  // namespace
 
-__global__ void __launch_bounds__(kVerifyWarps * 32) k_verify_hash(const uint8_t *arc, uint64_t arc_len,
-                                                                   const VerifyItem *items, int n, uint32_t *bad) {
-    __shared__ __align__(16) uint8_t s_tile[kVerifyWarps][kTileBuf];
-    const int w = threadIdx.x >> 5;
-    const int c = blockIdx.x * kVerifyWarps + w;
-    if (c >= n) return;   // whole warps leave together
-    uint8_t *tile = s_tile[w];
-    const VerifyItem it = items[c];
-    const uint8_t *blob = arc + it.co, *limit = arc + arc_len;
-    const uint16_t fml = (uint16_t)(blob[12] | (blob[13] << 8));
-    const uint8_t *fmap = blob + kBlobHdr, *bm = fmap + fml, *lens = bm + kBitmapBytes;
-    const uint64_t pay = (uint64_t)kBlobHdr + fml + kBitmapBytes + 2ull * it.np;
-    uint64_t h = xxh64_warp(arc, limit, fmap, fml, kHashSeed, tile);
-    h ^= xxh64_warp(arc, limit, bm, kBitmapBytes, h, tile);
-    h ^= xxh64_warp(arc, limit, lens, 2ull * it.np, h, tile);
-    h ^= xxh64_warp(arc, limit, blob + pay, it.len - pay, h, tile);
-    if ((threadIdx.x & 31) == 0) bad[c] = h != ld64u(blob + 4) ? 1u : 0u;
+// Device verify (src/mc_archive.c:1072-1111): the hash of every listed blob of
+// an archive held in device memory, compared with the hash stored in the
+// blob's header; bad[i] = 1 on a mismatch.
+__global__ void __launch_bounds__(kHashThreads) k_verify_hash(const uint8_t *arc, uint64_t arc_len,
+                                                              const VerifyItem *items, uint32_t *bad) {
+    __shared__ HashSmem S;
+    const VerifyItem it = items[blockIdx.x];
+    const uint8_t *blob = arc + it.co;
+    const uint64_t h = blob_hash_cta(arc, arc + arc_len, blob, it.len, it.np, S);
+    if (threadIdx.x == 0) bad[blockIdx.x] = h != ld64u(blob + 4) ? 1u : 0u;
 }
 
-// Hash chain per chunk blob (src/mc_archive.c:76-88), one warp per blob
-// through the same shared-memory tiles as the verify kernel; the hash goes
-// into the blob header.
-__global__ void __launch_bounds__(kVerifyWarps * 32) k_blob_hash(BlobParams P) {
-    __shared__ __align__(16) uint8_t s_tile[kVerifyWarps][kTileBuf];
-    const int w = threadIdx.x >> 5;
-    const int c = blockIdx.x * kVerifyWarps + w;
-    if (c >= P.nchunks) return;   // whole warps leave together
+// The hash of each assembled blob, 0 for an all-air chunk.
+__global__ void __launch_bounds__(kHashThreads) k_blob_hash(BlobParams P) {
+    __shared__ HashSmem S;
+    const int c = blockIdx.x;
     const uint64_t total = P.blob_len[c];
-    if (!total) return;
-    uint8_t *tile = s_tile[w];
-    uint8_t *blob = P.blobs + P.blob_off[c];
-    const uint8_t *limit = blob + total;
-    const uint16_t fml = (uint16_t)(blob[12] | (blob[13] << 8));
-    const uint8_t *fmap = blob + kBlobHdr, *bm = fmap + fml, *lens = bm + kBitmapBytes;
-    const uint32_t np = P.np[c];
-    const uint64_t pay = (uint64_t)kBlobHdr + fml + kBitmapBytes + 2ull * np;
-    uint64_t h = xxh64_warp(blob, limit, fmap, fml, kHashSeed, tile);
-    h ^= xxh64_warp(blob, limit, bm, kBitmapBytes, h, tile);
-    h ^= xxh64_warp(blob, limit, lens, 2ull * np, h, tile);
-    h ^= xxh64_warp(blob, limit, blob + pay, total - pay, h, tile);
-    if ((threadIdx.x & 31) == 0)
-        for (int i = 0; i < 8; ++i) blob[4 + i] = (uint8_t)(h >> (8 * i));
+    uint64_t h = 0;
+    if (total) {
+        const uint8_t *blob = P.blobs + P.blob_off[c];
+        h = blob_hash_cta(blob, blob + total, blob, total, P.np[c], S);
+    }
+    if (threadIdx.x == 0) P.hash[c] = h;
 }
 
 cudaError_t launch_verify_hash(const uint8_t *d_arc, uint64_t arc_len, const VerifyItem *d_items, int n,
                                uint32_t *d_bad, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_verify_hash<<<(unsigned)((n + kVerifyWarps - 1) / kVerifyWarps), kVerifyWarps * 32, 0, s>>>(d_arc, arc_len,
-                                                                                                d_items, n, d_bad);
+    k_verify_hash<<<(unsigned)n, kHashThreads, 0, s>>>(d_arc, arc_len, d_items, d_bad);
     return cudaGetLastError();
 }
 
@@ -675,13 +726,22 @@ cudaError_t launch_encode(const EncParams &p, cudaStream_t s) {
     });
     int blocks = p.n < sms * occ ? p.n : sms * occ;
     k_encode<<<blocks, 128, smem, s>>>(p);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_encode_rc(const EncParams &p, cudaStream_t s) {
+    if (p.n <= 0) return cudaSuccess;
+    const int sms = dev_sms();
     const int rc_blocks = (p.n + 127) / 128;
     k_encode_rc<<<rc_blocks < sms * 16 ? rc_blocks : sms * 16, 128, 0, s>>>(p);
     return cudaGetLastError();
 }
 
+cudaError_t launch_fracmap(const BlobParams &p, cudaStream_t s) {
+    if (p.nchunks <= 0) return cudaSuccess;
+    k_fracmap<<<p.nchunks, 32, 0, s>>>(p);
+    return cudaGetLastError();
+}
 cudaError_t launch_blob_layout(const BlobParams &p, cudaStream_t s) {
     if (p.nchunks <= 0) return cudaSuccess;
     k_blob_layout<<<p.nchunks, 1024, 0, s>>>(p);
@@ -694,7 +754,7 @@ cudaError_t launch_blob_fill(const BlobParams &p, cudaStream_t s) {
 }
 cudaError_t launch_blob_hash(const BlobParams &p, cudaStream_t s) {
     if (p.nchunks <= 0) return cudaSuccess;
-    k_blob_hash<<<(p.nchunks + kVerifyWarps - 1) / kVerifyWarps, kVerifyWarps * 32, 0, s>>>(p);
+    k_blob_hash<<<p.nchunks, kHashThreads, 0, s>>>(p);
     return cudaGetLastError();
 }
 

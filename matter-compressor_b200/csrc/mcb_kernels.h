@@ -171,7 +171,8 @@ struct EncParams {
     uint2 *sym;
 };
 cudaError_t upload_cos_encode(const float cmf[16][16], cudaStream_t s);
-cudaError_t launch_encode(const EncParams &p, cudaStream_t s);
+cudaError_t launch_encode(const EncParams &p, cudaStream_t s);      // transform: levels, corrections, nibbles
+cudaError_t launch_encode_rc(const EncParams &p, cudaStream_t s);   // range coder, after it
 
 // Chunk-blob assembly for chunks whose blocks were encoded by launch_encode
 // with items in block order (chunk c owns items [4096c, 4096c+4096)).
@@ -191,8 +192,10 @@ struct BlobParams {
     // write-pass inputs
     const uint64_t *blob_off; // per chunk: offset of the blob in `blobs`
     uint8_t *blobs;
+    uint64_t *hash;           // per chunk: the blob's chained xxh64 (the header's field stays 0)
 };
-cudaError_t launch_blob_layout(const BlobParams &p, cudaStream_t s);   // sizing pass
+cudaError_t launch_fracmap(const BlobParams &p, cudaStream_t s);       // fraction maps, after the transform
+cudaError_t launch_blob_layout(const BlobParams &p, cudaStream_t s);   // sizing pass, after both coders
 cudaError_t launch_blob_fill(const BlobParams &p, cudaStream_t s);     // write pass
 cudaError_t launch_blob_hash(const BlobParams &p, cudaStream_t s);     // xxh64 chain
 // Device verify: blob i at d_arc + co, `len` bytes, np present blocks; its

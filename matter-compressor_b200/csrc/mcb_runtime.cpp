@@ -144,6 +144,9 @@ Lane::~Lane() {
     for (cudaEvent_t e : bounce_ev)
         if (e) cudaEventDestroy(e);
     if (done) cudaEventDestroy(done);
+    if (ev_side) cudaEventDestroy(ev_side);
+    if (ev_main) cudaEventDestroy(ev_main);
+    if (side) cudaStreamDestroy(side);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -613,6 +616,13 @@ uint32_t lane_bad_blocks(Lane &L) {
 }
 
 // ------------------------------------------------------------------ encode
+static bool encode_streams(Lane &L) {
+    if (L.ev_main) return true;
+    return (L.side || cuda_ok(cudaStreamCreateWithFlags(&L.side, cudaStreamNonBlocking), "stream")) &&
+           (L.ev_side || cuda_ok(cudaEventCreateWithFlags(&L.ev_side, cudaEventDisableTiming), "event")) &&
+           cuda_ok(cudaEventCreateWithFlags(&L.ev_main, cudaEventDisableTiming), "event");
+}
+
 bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const float *header_q, const float *q,
                    const int *tau, std::vector<uint64_t> &blob_off, std::vector<uint64_t> &blob_len) {
     Runtime *R = runtime();
@@ -627,7 +637,8 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
         !L.status.ensure(16) || !L.b_scratch.ensure(4 * n) || !L.b_lens16.ensure(2 * n) ||
         !L.b_bitmap.ensure((size_t)kBitmapBytes * nchunks) || !L.b_fmap.ensure((size_t)kFmapCap * nchunks) ||
         !L.b_fml.ensure(4 * nchunks) || !L.b_np.ensure(4 * nchunks) || !L.b_len.ensure(8 * nchunks) ||
-        !L.b_off.ensure(8 * nchunks) || !L.b_q.ensure(4 * nchunks) || !L.h_misc.ensure(16 * (size_t)nchunks) ||
+        !L.b_off.ensure(8 * nchunks) || !L.b_q.ensure(4 * nchunks) || !L.h_misc.ensure(24 * (size_t)nchunks) ||
+        !L.b_hash.ensure(8 * (size_t)nchunks) || !encode_streams(L) ||
         !L.enc_lv.ensure(2 * (size_t)kN3 * n) || !L.enc_corr.ensure(4 * (size_t)kN3 * n) || !L.enc_sym.ensure(8 * n))
         return false;
     EncItem *hi = L.h_items.as<EncItem>();
@@ -663,7 +674,6 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
     ep.levels = L.enc_lv.as<int16_t>();
     ep.corr = L.enc_corr.as<uint32_t>();
     ep.sym = L.enc_sym.as<uint2>();
-    if (!cuda_ok(launch_encode(ep, L.stream), "encode launch")) return false;
     BlobParams bp;
     bp.nchunks = nchunks;
     bp.payload = L.enc_pay.as<uint8_t>();
@@ -679,7 +689,17 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
     bp.blob_len = L.b_len.as<uint64_t>();
     bp.blob_off = L.b_off.as<uint64_t>();
     bp.blobs = nullptr;
-    if (!cuda_ok(launch_blob_layout(bp, L.stream), "blob layout launch")) return false;
+    bp.hash = L.b_hash.as<uint64_t>();
+    // the fraction maps need the transform only: beside the block coder
+    if (!cuda_ok(launch_encode(ep, L.stream), "encode launch") ||
+        !cuda_ok(cudaEventRecord(L.ev_main, L.stream), "event record") ||
+        !cuda_ok(cudaStreamWaitEvent(L.side, L.ev_main, 0), "stream wait") ||
+        !cuda_ok(launch_fracmap(bp, L.side), "fraction map launch") ||
+        !cuda_ok(cudaEventRecord(L.ev_side, L.side), "event record") ||
+        !cuda_ok(launch_encode_rc(ep, L.stream), "range coder launch") ||
+        !cuda_ok(cudaStreamWaitEvent(L.stream, L.ev_side, 0), "stream wait") ||
+        !cuda_ok(launch_blob_layout(bp, L.stream), "blob layout launch"))
+        return false;
     uint64_t *hl = reinterpret_cast<uint64_t *>(L.h_misc.as<uint8_t>() + 8 * (size_t)nchunks);
     uint32_t status = 0;
     if (!cuda_ok(cudaMemcpyAsync(hl, L.b_len.p, 8 * (size_t)nchunks, cudaMemcpyDeviceToHost, L.stream), "D2H") ||
@@ -699,10 +719,21 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
     bp.blobs = L.blobs.as<uint8_t>();
     if (!cuda_ok(cudaMemcpyAsync(L.b_off.p, ho, 8 * (size_t)nchunks, cudaMemcpyHostToDevice, L.stream), "H2D") ||
         !cuda_ok(launch_blob_fill(bp, L.stream), "blob fill launch") ||
-        !cuda_ok(launch_blob_hash(bp, L.stream), "blob hash launch") ||
-        !cuda_ok(cudaStreamSynchronize(L.stream), "blob sync"))
+        !cuda_ok(cudaEventRecord(L.ev_main, L.stream), "event record") ||
+        !cuda_ok(cudaStreamWaitEvent(L.side, L.ev_main, 0), "stream wait") ||
+        !cuda_ok(launch_blob_hash(bp, L.side), "blob hash launch") ||
+        !cuda_ok(cudaMemcpyAsync(L.h_misc.as<uint8_t>() + 16 * (size_t)nchunks, L.b_hash.p, 8 * (size_t)nchunks,
+                                 cudaMemcpyDeviceToHost, L.side), "D2H hashes")) {
+        cudaStreamSynchronize(L.side);   // nothing of this call outlives it
+        cudaStreamSynchronize(L.stream);
         return false;
+    }
     return true;
+}
+
+const uint64_t *encode_hashes(Lane &L, int nchunks) {
+    if (!cuda_ok(cudaStreamSynchronize(L.side), "hash sync")) return nullptr;
+    return reinterpret_cast<const uint64_t *>(L.h_misc.as<uint8_t>() + 16 * (size_t)nchunks);
 }
 
 }  // namespace mcb

@@ -103,7 +103,9 @@ struct Lane {
     DecodeBatch batch;
     DevBuf enc_items, enc_len, enc_frac, enc_pay, src;
     DevBuf enc_lv, enc_corr, enc_sym;   // encoder symbol scratch (levels, corrections, per-block info)
-    DevBuf b_scratch, b_lens16, b_bitmap, b_fmap, b_fml, b_np, b_len, b_off, b_q, blobs;
+    DevBuf b_scratch, b_lens16, b_bitmap, b_fmap, b_fml, b_np, b_len, b_off, b_q, b_hash, blobs;
+    cudaStream_t side = nullptr;                // encoder: fraction maps beside the block coder, hashes beside the copy-out
+    cudaEvent_t ev_side = nullptr, ev_main = nullptr;
     DevBuf pyr_stage, pyr_a, pyr_b, pyr_flag;   // LOD pyramid: chunk staging, level volumes, all-air flags
     DevBuf ver_items, ver_bad;                  // device verify: blob list, mismatch flags
     DevBuf smp_grid, smp_cand, smp_acc;         // box sampling: block-fraction grid, candidates, accept flags
@@ -159,10 +161,15 @@ bool decode_one(Lane &L, const DecItem &it);
 bool decode_one_host(Lane &L, DecItem it, uint8_t *dst);
 
 // Encodes chunks of 256^3 voxels resident on the device (chunk c at
-// d_vox[c]) into assembled blobs. Synchronises; on return blob_len[c]
-// (0 = all air) and the blob offsets inside L.blobs are filled.
+// d_vox[c]) into assembled blobs. On return blob_len[c] (0 = all air) and the
+// blob offsets inside L.blobs are known; the blobs are complete, but for the
+// hash in their headers, behind the work on L.stream. Their hashes are on the
+// way to the host on L.side: encode_hashes waits for them and gives them
+// (nchunks values, valid until the next call on the lane). It must be called
+// before the lane encodes again.
 bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const float *header_q, const float *q,
                    const int *tau, std::vector<uint64_t> &blob_off, std::vector<uint64_t> &blob_len);
+const uint64_t *encode_hashes(Lane &L, int nchunks);
 
 // Blocks whose corrupt streams were cut short during the last decode on the lane.
 uint32_t lane_bad_blocks(Lane &L);
