@@ -446,7 +446,7 @@ int mc_enc_block(mc_codec_ctx *C, const mc_u8 *vox, mc_buf *out, uint32_t *len_o
     if (slot < 0) return 0;
     if (!cuda_ok(cudaEventSynchronize(L->done), "sync") || !L->src.ensure(kN3) || !L->enc_pay.ensure(kEncCap) ||
         !L->enc_len.ensure(4) || !L->enc_frac.ensure(4) || !L->enc_items.ensure(sizeof(EncItem)) ||
-        !L->status.ensure(16) || !L->h_stage.ensure(kEncCap + 64) || !L->enc_lv.ensure(2 * kN3) ||
+        !L->status.ensure(16) || !L->h_stage.ensure(kEncCap + 64) || !L->enc_ent.ensure(4 * kN3) ||
         !L->enc_corr.ensure(4 * kN3) || !L->enc_sym.ensure(8))
         return 0;
     EncItem it{};
@@ -467,7 +467,7 @@ int mc_enc_block(mc_codec_ctx *C, const mc_u8 *vox, mc_buf *out, uint32_t *len_o
     ep.len = L->enc_len.as<uint32_t>();
     ep.frac = L->enc_frac.as<uint8_t>();
     ep.status = L->status.as<uint32_t>();
-    ep.levels = L->enc_lv.as<int16_t>();
+    ep.entries = L->enc_ent.as<uint32_t>();
     ep.corr = L->enc_corr.as<uint32_t>();
     ep.sym = L->enc_sym.as<uint2>();
     uint32_t len = 0;

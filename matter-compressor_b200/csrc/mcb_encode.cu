@@ -1,14 +1,15 @@
 // mcb_encode.cu -- sm_100a block encode and chunk-blob assembly.
 //
 // k_encode: one CTA (128 threads) per 16^3 block (src/mc_codec.c:629-736).
-//   gather + sum/count -> dc, material nibble -> forward DCT-II along x, y, z
+//   gather + sum/count -> dc -> forward DCT-II along x, y, z
 //   (each output a sequential single-precision sum over n of the even/odd
 //   halves, src/mc_codec_float.h:83-95) -> fused dead-zone quantiser
 //   (src/mc_codec.c:686-692) -> optional max-error pass: dequantise, inverse
 //   transform, lrint + dc, list every voxel whose error exceeds tau
-//   (:697-708) -> range coding of header bins, coefficients and corrections
-//   by one thread (the coder is a serial chain; src/mc_codec.c:178-233).
-// k_fracmap / k_blob_layout / k_blob_fill / k_blob_hash: per-chunk blob assembly
+//   (:697-708) -> the block's symbols in scratch.
+// k_encode_rc: range coding of header bins, coefficients and corrections, one
+//   lane per block (the coder is a serial chain; src/mc_codec.c:178-233).
+// k_frac_count / k_fracmap / k_blob_layout / k_blob_fill / k_blob_hash: per-chunk blob assembly
 //   (src/mc_codec.c:809-845, src/mc_archive.c:861-901): bitmap + u16 lengths
 //   in block order, fraction map range-coded (src/mc_codec.c:600-611),
 //   payloads concatenated in block order, xxh64 chain over
@@ -22,7 +23,10 @@
 
 namespace mcb {
 
-__constant__ float c_cos[16][16];   // this translation unit's copy (no -rdc)
+// this translation unit's copies (no -rdc): the cosine basis, and the first scan
+// position past each band (b < 7), then kN3 and a sentinel
+__constant__ float c_cos[16][16];
+__constant__ uint16_t c_bend[9];
 
 namespace {
 
@@ -59,43 +63,7 @@ __device__ __forceinline__ void enc_shift(Enc &e) {
 __device__ __forceinline__ void enc_norm(Enc &e) {
     while (e.range < (1u << 24)) { enc_shift(e); e.range <<= 8; }
 }
-__device__ __forceinline__ void enc_bit(Enc &e, uint16_t &p0, uint32_t bit) {
-    uint32_t r0 = (e.range >> 12) * (uint32_t)p0;
-    if (!bit) { e.range = r0; p0 = (uint16_t)(p0 + ((4096u - p0) >> 4)); }
-    else { e.low += r0; e.range -= r0; p0 = (uint16_t)(p0 - (p0 >> 4)); }
-    enc_norm(e);
-}
-__device__ __forceinline__ void enc_bypass(Enc &e, uint32_t bit) {
-    e.range >>= 1;
-    if (bit) e.low += e.range;
-    enc_norm(e);
-}
-// k bits MSB-first, 16 at a time from the top (src/mc_codec.c:209-215)
-__device__ void enc_bits(Enc &e, uint32_t v, int k) {
-    int chunks = k > 16 ? (k - 1) / 16 : 0;    // leading 16-bit pieces
-    for (int c = chunks; c > 0; --c) {
-        int sh = k - 16;
-        uint32_t piece = (sh >= 32 ? 0u : (v >> sh)) & 0xFFFFu;
-        e.range >>= 16;
-        e.low += (uint64_t)piece * e.range;
-        enc_norm(e);
-        k -= 16;
-    }
-    if (k == 0) return;
-    e.range >>= k;
-    e.low += (uint64_t)(v & ((1u << k) - 1u)) * e.range;
-    enc_norm(e);
-}
 __device__ __forceinline__ int bitlen32(uint32_t v) { return v ? 32 - __clz(v) : 0; }
-// order-0 Exp-Golomb (src/mc_codec.c:229-233)
-__device__ void enc_eg(Enc &e, uint32_t v) {
-    uint32_t t = v + 1u;
-    int nb = t ? bitlen32(t) - 1 : 0;
-    for (int i = 0; i < nb; ++i) enc_bypass(e, 1);
-    enc_bypass(e, 0);
-    if (nb) enc_bits(e, (v + 1u) & ((1u << nb) - 1u), nb);
-}
-
 // ------------------------------------------------------------ transforms
 // forward DCT-II, outputs k in {j, j+4, j+8, j+12} of one line
 __device__ __forceinline__ void fdct_quad(const float *in, int si, float *out, int so, int j) {
@@ -169,7 +137,7 @@ struct EncSmem {
     float b[kN3];
     int16_t lv[kN3];
     uint8_t vox[kN3];
-    uint32_t mask[4][32];   // max-error pass: hit masks per warp and step
+    uint32_t mask[4][32];   // entry list and max-error pass: hit masks per warp and step
     uint32_t red[8];
     uint32_t ncorr;
     uint32_t eob;
@@ -222,12 +190,7 @@ __global__ void __launch_bounds__(128) k_encode(EncParams P) {
         __syncthreads();
         sum = S.red[0] + S.red[1] + S.red[2] + S.red[3];
         cnt = S.red[4] + S.red[5] + S.red[6] + S.red[7];
-        if (tid == 0) {
-            uint32_t f = (cnt * 15u + 2048u) / 4096u;    // material nibble (src/mc_codec.c:820-822)
-            if (cnt && !f) f = 1;
-            P.frac[item] = (uint8_t)f;
-            if (!cnt) { P.len[item] = 0; P.sym[item] = make_uint2(0, 0); }
-        }
+        if (tid == 0 && !cnt) { P.len[item] = 0; P.sym[item] = make_uint2(0, 0); }
         if (!cnt) { __syncthreads(); continue; }       // all air: not coded
         const int dc = (int)((sum + kN3 / 2) / kN3);
         for (int i = tid; i < kN3; i += 128) S.a[i] = (float)((int)S.vox[i] - dc);
@@ -246,11 +209,36 @@ __global__ void __launch_bounds__(128) k_encode(EncParams P) {
             S.lv[i] = (int16_t)(c < 0.0f ? -v : v);
         }
         __syncthreads();
-        // eob = 1 + last scan position holding a nonzero level
-        for (int p = tid; p < kN3; p += 128)
-            if (S.lv[__ldg(P.scan + p) & 0xFFF]) last = max(last, (uint32_t)p + 1);
-        for (int o = 16; o; o >>= 1) last = max(last, __shfl_xor_sync(0xFFFFFFFFu, last, o));
-        if ((tid & 31) == 0) atomicMax(&S.eob, last);
+        // the nonzero levels in scan order as one entry list (position | level
+        // << 16) for k_encode_rc: warp w owns positions [1024w, 1024w + 1024) in
+        // 32 steps of 32; a first pass counts (the step masks kept in shared
+        // memory), one barrier gives every warp its start, a second pass writes
+        {
+            const int lane = tid & 31, w = tid >> 5;
+            uint32_t cnt_w = 0;
+            for (int k = 0; k < 32; ++k) {
+                const uint32_t p0 = 1024u * w + 32u * k;
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, S.lv[__ldg(P.scan + p0 + lane) & 0xFFF] != 0);
+                if (lane == 0) S.mask[w][k] = m;
+                cnt_w += __popc(m);
+                if (m) last = p0 + 32u - __clz(m);   // eob = 1 + last nonzero position
+            }
+            if (lane == 0) {
+                S.red[w] = cnt_w;
+                atomicMax(&S.eob, last);
+            }
+            __syncthreads();
+            uint32_t at = 0;
+            for (int ww = 0; ww < w; ++ww) at += S.red[ww];
+            uint32_t *ent = P.entries + (size_t)item * kN3;
+            for (int k = 0; k < 32; ++k) {
+                const uint32_t m = S.mask[w][k], p = 1024u * w + 32u * k + lane;
+                if ((m >> lane) & 1)
+                    ent[at + __popc(m & ((1u << lane) - 1u))] =
+                        p | (uint32_t)(uint16_t)S.lv[__ldg(P.scan + p) & 0xFFF] << 16;
+                at += __popc(m);
+            }
+        }
         if (it.tau > 0) {
             // local reconstruction for the max-error pass
             for (int i = tid; i < kN3; i += 128) {
@@ -298,13 +286,9 @@ __global__ void __launch_bounds__(128) k_encode(EncParams P) {
             }
             if (tid == 0) S.ncorr = S.red[0] + S.red[1] + S.red[2] + S.red[3];
         }
-        __syncthreads();   // eob (per-warp atomics) and ncorr complete
-        // the block's symbols for k_encode_rc: levels in scan order up to the
-        // EOB, the corrections, and (dc, eob, ncorr) with the coded flag
-        const uint32_t eob = S.eob, ncorr = S.ncorr;
-        int16_t *lvs = P.levels + (size_t)item * kN3;
-        for (uint32_t p = tid; p < eob; p += 128) lvs[p] = S.lv[__ldg(P.scan + p) & 0xFFF];
-        if (tid == 0) P.sym[item] = make_uint2(0x80000000u | (eob << 8) | (uint32_t)dc, ncorr);
+        __syncthreads();   // ncorr complete
+        // (dc, eob) with the coded flag, ncorr
+        if (tid == 0) P.sym[item] = make_uint2(0x80000000u | (S.eob << 8) | (uint32_t)dc, S.ncorr);
         __syncthreads();
     }
 }
@@ -313,76 +297,345 @@ __global__ void __launch_bounds__(128) k_encode(EncParams P) {
 // 330-350, 710-729): header bins, EOB, the coefficient loop and the
 // corrections, in the order the reference writes them. The coder of a block is
 // a serial chain; lanes in a warp code different blocks, with contexts in
-// shared memory (one 16-bit word per context per lane).
-__global__ void __launch_bounds__(128) k_encode_rc(EncParams P) {
-    __shared__ uint16_t s_ctx[4][kNumCtx][32];
+// shared memory (one word per context per lane, context j of lane l at word
+// j * 32 + l).
+//
+// The coefficient loop is the mirror of the decoder's (k_entropy in
+// mcb_decode.cu): one step of straight-line code advances every lane by a run of
+// one or four zeros, a significance bin, a magnitude rung and a sign. A run of
+// zeros does not touch the code value and the range only falls, so the last
+// split above the renormalisation bound says that none of the run renormalises.
+//
+// The code value is `low` with its not yet written bytes in front of it
+// (ah:al, n of them, at least two), so that a carry ripples through by plain
+// addition; the bytes go out two at a time, and a carry past all of them, about
+// one in 65536 writes, walks back through the bytes already written.
+namespace {
+constexpr int kEncSlots = kNumCtx + 1;   // one more: 1, the "probability" of a bypass bin (see k_entropy)
+constexpr uint32_t kEncScr = kNumCtx;
+constexpr uint32_t kEncTop = 1u << 24;
+
+struct EncLane {
+    uint8_t *out;
+    uint32_t len;                   // bytes written
+    uint32_t n, ah, al, low, range;
+    const uint32_t *ent;            // the block's entries
+    uint32_t idx, ahead;            // next entry to load, the entry after the current one
+    uint32_t pos, m, neg, kend;     // current coefficient: position, magnitude, sign, one-bits of its unary code
+    uint32_t p, eob, sigb, band, bend, stop;
+    uint32_t e1, e2, e3;            // the last three significant positions + 17, newest first
+    uint32_t cs, ps, lim;           // context slot at p, its probability, where either changes
+    uint32_t k, pm;                 // next rung (0 at a significance bin), its probability
+    bool live;
+};
+
+__device__ __forceinline__ void code_add(EncLane &e, uint32_t v) {
+    const uint32_t t = e.low + v, a = e.al + (t < v ? 1u : 0u);
+    e.ah += a < e.al ? 1u : 0u;
+    e.al = a;
+    e.low = t;
+}
+// Bits that a renormalisation shifts out: 0, 8 or 16 (src/mc_codec.c:180-187)
+__device__ __forceinline__ uint32_t code_norm(EncLane &e) {
+    const uint32_t s = e.range < (1u << 16) ? 16u : (e.range < kEncTop ? 8u : 0u);
+    e.ah = funnel_left(e.al, e.ah, s);
+    e.al = funnel_left(e.low, e.al, s);
+    e.low <<= s;
+    e.range <<= s;
+    e.n += s >> 3;
+    return s;
+}
+__device__ __forceinline__ void put_byte(EncLane &e, uint32_t b) {
+    if (e.len < (uint32_t)kEncCap) e.out[e.len] = (uint8_t)b;
+    ++e.len;
+}
+// A carry past the held bytes: one more in the bytes already written.
+__device__ __noinline__ void code_carry(uint8_t *out, uint32_t len) {
+    uint32_t i = min(len, (uint32_t)kEncCap);
+    while (i > 0 && ++out[i - 1] == 0) --i;
+}
+// Writes the two oldest of n >= 4 held bytes.
+__device__ __forceinline__ void code_flush(EncLane &e) {
+    uint64_t acc = (uint64_t)e.ah << 32 | e.al;
+    const uint32_t sh = 8u * (e.n - 2u);   // 16..40
+    const uint32_t v = (uint32_t)(acc >> sh);
+    acc &= (1ull << sh) - 1u;
+    e.ah = (uint32_t)(acc >> 32);
+    e.al = (uint32_t)acc;
+    e.n -= 2;
+    if (v >> 16) code_carry(e.out, e.len);
+    if (e.len + 2 <= (uint32_t)kEncCap)   // even offsets, even base
+        *reinterpret_cast<uint16_t *>(e.out + e.len) = (uint16_t)((v >> 8 & 0xFFu) | (v & 0xFFu) << 8);
+    e.len += 2;
+}
+__device__ __forceinline__ void code_settle(EncLane &e) {   // after a single operation
+    code_norm(e);
+    while (e.range < kEncTop) code_norm(e);
+    while (e.n >= 4) code_flush(e);
+}
+__device__ __forceinline__ void code_bin(EncLane &e, uint32_t *c, uint32_t bit) {
+    const uint32_t p0 = *c, r0 = (e.range >> 12) * p0;
+    if (!bit) { e.range = r0; *c = p0 + ((4096u - p0) >> 4); }
+    else { code_add(e, r0); e.range -= r0; *c = p0 - (p0 >> 4); }
+    code_settle(e);
+}
+__device__ __forceinline__ void code_bypass(EncLane &e, uint32_t bit) {
+    e.range >>= 1;
+    if (bit) code_add(e, e.range);
+    code_settle(e);
+}
+// k bits MSB-first, 16 at a time from the top (src/mc_codec.c:209-215)
+__device__ __forceinline__ void code_bits(EncLane &e, uint32_t v, int k) {
+    while (k > 0) {
+        const int take = k > 16 ? 16 : k;
+        e.range >>= take;
+        code_add(e, ((v >> (k - take)) & ((1u << take) - 1u)) * e.range);
+        code_settle(e);
+        k -= take;
+    }
+}
+// order-0 Exp-Golomb (src/mc_codec.c:229-233)
+__device__ __forceinline__ void code_eg(EncLane &e, uint32_t v) {
+    const uint32_t t = v + 1u;
+    const int nb = bitlen32(t) - 1;
+    for (int i = 0; i < nb; ++i) code_bypass(e, 1);
+    code_bypass(e, 0);
+    if (nb > 0) code_bits(e, t & ((1u << nb) - 1u), nb);
+}
+
+__device__ __forceinline__ void enc_density(EncLane &e) {
+    const bool a3 = e.p < e.e3, a2 = e.p < e.e2, a1 = e.p < e.e1;
+    e.cs = e.sigb + (a3 ? 3u : (a2 ? 2u : (a1 ? 1u : 0u)));
+    e.lim = min(e.stop, a3 ? e.e3 : (a2 ? e.e2 : (a1 ? e.e1 : 0xFFFFFFFFu)));
+}
+__device__ __forceinline__ void set_entry(EncLane &e, uint32_t w) {
+    const int lv = (int)w >> 16;
+    e.pos = w & 0xFFFFu;
+    e.neg = lv < 0 ? 1u : 0u;
+    e.m = (uint32_t)(lv < 0 ? -lv : lv);
+    // m - 1 ones and a zero up to m = 12; twelve ones and the prefix of the
+    // Exp-Golomb code of m - 12 beyond (src/mc_codec.c:268-275)
+    e.kend = e.m <= 12u ? e.m - 1u : 43u - (uint32_t)__clz(e.m - 11u);
+}
+__device__ __forceinline__ void next_entry(EncLane &e) {
+    set_entry(e, e.ahead);
+    e.ahead = e.ent[min(e.idx, (uint32_t)kN3 - 1u)];
+    ++e.idx;
+}
+// p >= stop: a band change, or the last position, significant by definition:
+// its coefficient without a significance bin (src/mc_codec.c:337-349); the
+// coefficient loop is then over.
+__device__ __forceinline__ void enc_position(EncLane &e, uint32_t *ctx, const uint16_t *s_bend) {
+    while (e.p >= e.bend) { e.band++; e.sigb += 4; e.bend = s_bend[e.band]; }
+    if (e.p + 1 >= e.eob) {
+        for (uint32_t k = 0; k < 12u; ++k) {
+            code_bin(e, ctx + (kCtxMag + k) * 32, k < e.kend);
+            if (k >= e.kend) break;
+        }
+        if (e.m > 12u) code_eg(e, e.m - 12u);
+        code_bypass(e, e.neg);
+        e.live = false;
+        e.lim = e.stop = 0xFFFFFFFFu;
+        return;
+    }
+    e.stop = min(e.bend, e.eob - 1);
+    enc_density(e);
+    e.ps = ctx[e.cs * 32];
+}
+
+// One step of every live lane; returns whether enc_event has work for the lane.
+__device__ __forceinline__ bool enc_step(EncLane &e, uint32_t *ctx, bool &rest) {
+    const uint32_t k0 = e.k;
+    const bool is_sig = e.live & (k0 == 0u);
+    uint32_t pr = e.ps, p = e.p;
+    {   // zeros
+        const uint32_t gap = e.pos - p, room = is_sig ? min(e.lim - p, gap + 1u) : 0u;
+        const uint32_t r1 = (e.range >> 12) * pr, q1 = (15u * pr + 4096u) >> 4;
+        const uint32_t r2 = (r1 >> 12) * q1, q2 = (15u * q1 + 4096u) >> 4;
+        const uint32_t r3 = (r2 >> 12) * q2, q3 = (15u * q2 + 4096u) >> 4;
+        const uint32_t r4 = (r3 >> 12) * q3, q4 = (15u * q3 + 4096u) >> 4;
+        const bool z1 = (r1 >= kEncTop) & (room > 1u), z4 = (r4 >= kEncTop) & (room > 4u);
+        e.range = z4 ? r4 : (z1 ? r1 : e.range);
+        pr = z4 ? q4 : (z1 ? q1 : pr);
+        p += z4 ? 4u : (z1 ? 1u : 0u);
+    }
+    // the significance bin at p
+    const bool one = is_sig & (p == e.pos);
+    const uint32_t r1 = is_sig ? (e.range >> 12) * pr : e.range;
+    code_add(e, one ? r1 : 0u);
+    e.range = one ? e.range - r1 : r1;
+    if (is_sig) ctx[e.cs * 32] = (15u * pr + (one ? 15u : 4096u)) >> 4;
+    const uint32_t s1 = code_norm(e);
+    p += is_sig ? 1u : 0u;
+    e.p = p;
+    e.e3 = one ? e.e2 : e.e3;
+    e.e2 = one ? e.e1 : e.e2;
+    e.e1 = one ? p + 16u : e.e1;
+    enc_density(e);
+    e.ps = ctx[e.cs * 32];
+    // a rung, or a bit of the prefix behind the twelfth
+    const bool act = one | (k0 != 0u), pfx = k0 >= 12u;
+    const bool up = act & (k0 < e.kend);
+    const uint32_t pm = e.pm;
+    const uint32_t r2 = act ? (e.range >> (pfx ? 1u : 12u)) * pm : e.range;
+    code_add(e, up ? r2 : 0u);
+    e.range = up & !pfx ? e.range - r2 : r2;
+    if (act & !pfx) ctx[(kCtxMag + k0) * 32] = (15u * pm + (up ? 15u : 4096u)) >> 4;
+    const uint32_t kn = up ? k0 + 1u : 0u;
+    e.k = kn;
+    e.pm = ctx[(kCtxMag + min(kn, 12u)) * 32];
+    const uint32_t s2 = code_norm(e);
+    // the sign, unless a suffix comes first or the held bytes are many
+    const bool closed = act & !up;
+    const bool sign = closed & !pfx & (s1 + s2 <= 16u);
+    const uint32_t r3 = sign ? e.range >> 1 : e.range;
+    code_add(e, (sign & (e.neg != 0u)) ? r3 : 0u);
+    e.range = r3;
+    code_norm(e);
+    if (sign) next_entry(e);
+    while (e.n >= 4) code_flush(e);
+    rest = closed & !sign;
+    return rest | (e.live & (kn == 0u) & (p >= e.stop));
+}
+__device__ __forceinline__ void enc_event(EncLane &e, uint32_t *ctx, const uint16_t *s_bend, bool rest) {
+    if (rest) {   // the suffix of an escape, the sign
+        if (e.m > 12u) {
+            const int nb = bitlen32(e.m - 11u) - 1;
+            code_bits(e, (e.m - 11u) & ((1u << nb) - 1u), nb);
+        }
+        code_bypass(e, e.neg);
+        next_entry(e);
+    }
+    if (e.p >= e.stop) enc_position(e, ctx, s_bend);
+}
+}  // namespace
+
+// Warp groups of `lanes` blocks (the warp's other lanes idle): launches of few
+// blocks spread them over more warps, since a warp's time is its longest
+// block's chain and its lanes' rare events add up.
+constexpr int kRcWarps = 4;
+__global__ void __launch_bounds__(kRcWarps * 32) k_encode_rc(EncParams P, int lanes) {
+    __shared__ uint32_t s_ctx[kRcWarps][kEncSlots][32];
+    __shared__ uint16_t s_bend[9];
+    if (threadIdx.x < 9) s_bend[threadIdx.x] = c_bend[threadIdx.x];
+    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint16_t *ctx = &s_ctx[warp][0][lane];
-    for (int item = blockIdx.x * blockDim.x + threadIdx.x; item < P.n; item += gridDim.x * blockDim.x) {
-        const uint2 sy = P.sym[item];
-        if (!(sy.x & 0x80000000u)) continue;   // all air: not coded
-        const EncItem it = P.items[item];
-        const QTab &qt = P.qtab[it.qslot];
+    uint32_t *ctx = &s_ctx[warp][0][lane];
+    const int ngroups = (P.n + lanes - 1) / lanes;
+    for (int g = blockIdx.x * kRcWarps + warp; g < ngroups; g += gridDim.x * kRcWarps) {
+        const int item = g * lanes + lane;
+        uint2 sy = make_uint2(0, 0);
+        if (lane < lanes && item < P.n) sy = P.sym[item];
+        const bool coded = (sy.x & 0x80000000u) != 0;   // an all-air block is not coded
         const uint32_t dc = sy.x & 0xFF, eob = (sy.x >> 8) & 0x1FFF, ncorr = sy.y;
-        const int16_t *lvs = P.levels + (size_t)item * kN3;
-        const uint32_t *cor = P.corr + (size_t)item * kN3;
-        Enc e;
-        e.out = reinterpret_cast<uint8_t *>(it.out);
-        e.cap = kEncCap; e.len = 0; e.low = 0; e.range = 0xFFFFFFFFu; e.cache = 0; e.pending = 1;
-        for (int j = 0; j < kNumCtx; ++j) ctx[j * 32] = qt.ctx[j];
-        enc_bit(e, ctx[(kCtxFlag + 0) * 32], 0);                 // reserved
-        enc_bit(e, ctx[(kCtxFlag + 1) * 32], ncorr > 0);
-        for (int b = 0; b < 8; ++b) enc_bit(e, ctx[(kCtxDc + b) * 32], (dc >> (7 - b)) & 1);
-        {   // EOB: bit length prefix then the bits below the MSB (src/mc_codec.c:314-320)
-            int k = bitlen32(eob);
-            for (int i = 0; i < k; ++i) enc_bit(e, ctx[(kCtxEob + i) * 32], 1);
-            if (k < 13) enc_bit(e, ctx[(kCtxEob + k) * 32], 0);
-            if (k > 1) enc_bits(e, eob & ((1u << (k - 1)) - 1u), k - 1);
-        }
-        uint32_t hist = 0;
-        for (uint32_t p = 0; p < eob; ++p) {              // src/mc_codec.c:337-349
-            const int v = lvs[p];
-            if (p != eob - 1) {
-                const uint32_t dens = min(__popc(hist & 0xFFFFu), 3);
-                enc_bit(e, ctx[(kCtxSig + (__ldg(P.scan + p) >> 12) * 4 + dens) * 32], v != 0);
-            }
-            hist = (hist << 1) | (v != 0);
-            if (!v) continue;
-            uint32_t m = (uint32_t)(v < 0 ? -v : v), rest = m - 1;
-            int k = 0;
-            while (rest > 0 && k < 11) { enc_bit(e, ctx[(kCtxMag + k) * 32], 1); rest--; k++; }
-            if (rest == 0) enc_bit(e, ctx[(kCtxMag + k) * 32], 0);
-            else { enc_bit(e, ctx[(kCtxMag + 11) * 32], 1); enc_eg(e, rest); }
-            enc_bypass(e, v < 0);
-        }
-        if (ncorr) {                                     // src/mc_codec.c:721-729
-            enc_eg(e, ncorr - 1);
-            uint32_t prev = 0;
-            for (uint32_t c = 0; c < ncorr; ++c) {
-                const uint32_t w = cor[c];
-                const uint32_t pos = w & 0xFFFF;
-                enc_eg(e, pos - prev);
-                prev = pos;
-                const int d = (int16_t)(w >> 16);
-                enc_bypass(e, d < 0);
-                enc_eg(e, (uint32_t)(d < 0 ? -d : d) - 1u);
+        EncLane e;
+        memset(&e, 0, sizeof e);
+        e.range = 0xFFFFFFFFu;
+        e.n = 1;   // the coder's leading byte
+        e.cs = e.sigb = kEncScr;
+        e.lim = e.stop = 0xFFFFFFFFu;
+        e.pm = 1;
+        if (coded) {
+            const EncItem it = P.items[item];
+            const QTab &qt = P.qtab[it.qslot];
+            e.out = reinterpret_cast<uint8_t *>(it.out);
+            for (int j = 0; j < kNumCtx; ++j) ctx[j * 32] = qt.ctx[j];
+            ctx[kEncScr * 32] = 1;
+            code_bin(e, ctx + (kCtxFlag + 0) * 32, 0);                 // reserved
+            code_bin(e, ctx + (kCtxFlag + 1) * 32, ncorr > 0);
+            for (int b = 0; b < 8; ++b) code_bin(e, ctx + (kCtxDc + b) * 32, (dc >> (7 - b)) & 1);
+            // EOB: bit length prefix then the bits below the MSB (src/mc_codec.c:314-320)
+            const int k = bitlen32(eob);
+            for (int i = 0; i < k; ++i) code_bin(e, ctx + (kCtxEob + i) * 32, 1);
+            if (k < 13) code_bin(e, ctx + (kCtxEob + k) * 32, 0);
+            if (k > 1) code_bits(e, eob & ((1u << (k - 1)) - 1u), k - 1);
+            if (eob) {
+                e.ent = P.entries + (size_t)item * kN3;
+                e.eob = eob;
+                e.sigb = kCtxSig;
+                e.bend = s_bend[0];
+                e.ahead = e.ent[0];
+                e.idx = 1;
+                next_entry(e);
+                e.live = true;
+                e.pm = ctx[kCtxMag * 32];
+                enc_position(e, ctx, s_bend);
             }
         }
-        for (int i = 0; i < 5; ++i) enc_shift(e);
-        if (e.len > e.cap) atomicAdd(P.status, 1u);
-        P.len[item] = e.len > e.cap ? e.cap : e.len;
+        __syncwarp();
+        while (__any_sync(0xFFFFFFFFu, e.live)) {
+            bool rest;
+            const bool ev = enc_step(e, ctx, rest);
+            if (__any_sync(0xFFFFFFFFu, ev)) {
+                if (ev) enc_event(e, ctx, s_bend, rest);
+                __syncwarp();
+            }
+        }
+        if (coded) {
+            if (ncorr) {                                     // src/mc_codec.c:721-729
+                const uint32_t *cor = P.corr + (size_t)item * kN3;
+                code_eg(e, ncorr - 1);
+                uint32_t prev = 0;
+                for (uint32_t c = 0; c < ncorr; ++c) {
+                    const uint32_t w = cor[c];
+                    const uint32_t pos = w & 0xFFFF;
+                    code_eg(e, pos - prev);
+                    prev = pos;
+                    const int d = (int16_t)(w >> 16);
+                    code_bypass(e, d < 0);
+                    code_eg(e, (uint32_t)(d < 0 ? -d : d) - 1u);
+                }
+            }
+            // the held bytes, then the four of low
+            const uint64_t acc = (uint64_t)e.ah << 32 | e.al;
+            if ((acc >> (8 * e.n)) & 1) code_carry(e.out, e.len);
+            for (int i = (int)e.n - 1; i >= 0; --i) put_byte(e, (uint32_t)(acc >> (8 * i)) & 0xFFu);
+            for (int i = 3; i >= 0; --i) put_byte(e, (e.low >> (8 * i)) & 0xFFu);
+            if (e.len > (uint32_t)kEncCap) atomicAdd(P.status, 1u);
+            P.len[item] = min(e.len, (uint32_t)kEncCap);
+        }
+        __syncwarp();
     }
 }
 
 // ------------------------------------------------------------ blob assembly
+// Material nibble of every block (src/mc_codec.c:820-822), one warp per block:
+// the voxels are read once more (20 us for 8 chunks) so that the fraction maps
+// need not wait for the transform.
+__global__ void __launch_bounds__(256) k_frac_count(EncParams P) {
+    const int item = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (item >= P.n) return;   // whole warps leave together
+    const EncItem it = P.items[item];
+    const uint8_t *src = reinterpret_cast<const uint8_t *>(it.src);
+    uint32_t cnt = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int r = j * 32 + lane;
+        const uint8_t *row = src + (r >> 4) * it.sz + (r & 15) * it.sy;
+        if (((uintptr_t)row & 15) == 0) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row));
+            cnt += __popc(__vsetne4(v.x, 0)) + __popc(__vsetne4(v.y, 0)) + __popc(__vsetne4(v.z, 0)) +
+                   __popc(__vsetne4(v.w, 0));
+        } else {
+            for (int x = 0; x < 16; ++x) cnt += row[x] != 0;
+        }
+    }
+    cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
+    if (lane == 0) {
+        uint32_t f = (cnt * 15u + 2048u) / 4096u;
+        if (cnt && !f) f = 1;
+        P.frac[item] = (uint8_t)f;
+    }
+}
+
 // Fraction map of a chunk, range-coded by one thread (src/mc_codec.c:600-611):
-// a chain of 16384 bins, which needs only the transform's material nibbles, so
-// it runs on a stream of its own beside the block coder. Most nibbles repeat
+// a chain of 16384 bins, which needs only the material nibbles, so it runs on a
+// stream of its own beside the transform and the block coder. Most nibbles repeat
 // one of the two extremes, air behind air (four 0 bins) or full behind full
 // (four 1 bins); such a nibble is coded straight through, the four splits
 // computed one from the other, when the last range shows that none of them
 // renormalises. One chunk or many: 0.95 ms as the tail of the sizing pass with
-// contexts in local memory, 0.75 ms here, beside the coder.
+// contexts in local memory, 0.75 ms here and hidden.
 __device__ __forceinline__ uint32_t up0(uint32_t p) { return p + ((4096u - p) >> 4); }
 __device__ __forceinline__ uint32_t up1(uint32_t p) { return p - (p >> 4); }
 __device__ __forceinline__ void frac_bit(Enc &e, uint32_t &p0, uint32_t bit) {
@@ -695,8 +948,17 @@ cudaError_t launch_verify_hash(const uint8_t *d_arc, uint64_t arc_len, const Ver
     return cudaGetLastError();
 }
 
-cudaError_t upload_cos_encode(const float cmf[16][16], cudaStream_t s) {
-    return cudaMemcpyToSymbolAsync(c_cos, cmf, sizeof(float) * 256, 0, cudaMemcpyHostToDevice, s);
+cudaError_t upload_encode_tables(const float cmf[16][16], const uint16_t scan[kN3], cudaStream_t s) {
+    // pageable sources: the copies are staged before these calls return
+    uint16_t bend[9];
+    for (int i = 1; i < kN3; ++i) {
+        const uint32_t b = scan[i] >> 12;
+        if ((uint32_t)(scan[i - 1] >> 12) != b) bend[b - 1] = (uint16_t)i;
+    }
+    bend[7] = kN3;
+    bend[8] = 0xFFFF;
+    const cudaError_t e = cudaMemcpyToSymbolAsync(c_cos, cmf, sizeof(float) * 256, 0, cudaMemcpyHostToDevice, s);
+    return e != cudaSuccess ? e : cudaMemcpyToSymbolAsync(c_bend, bend, sizeof bend, 0, cudaMemcpyHostToDevice, s);
 }
 
 cudaError_t launch_encode(const EncParams &p, cudaStream_t s) {
@@ -731,14 +993,22 @@ cudaError_t launch_encode(const EncParams &p, cudaStream_t s) {
 
 cudaError_t launch_encode_rc(const EncParams &p, cudaStream_t s) {
     if (p.n <= 0) return cudaSuccess;
+    // at least one warp for each of the SMs' four schedulers while a warp
+    // still has four blocks or more (8 chunks at q=6: 0.97 ms with 32 lanes, 1.36
+    // with 16; 2 chunks at q=1 tau=4: 5.06, 4.41, and 4.39 with 8)
     const int sms = dev_sms();
-    const int rc_blocks = (p.n + 127) / 128;
-    k_encode_rc<<<rc_blocks < sms * 16 ? rc_blocks : sms * 16, 128, 0, s>>>(p);
+    int lanes = 32;
+    while (lanes > 4 && p.n < lanes * sms * 4) lanes >>= 1;
+    const int blocks = ((p.n + lanes - 1) / lanes + kRcWarps - 1) / kRcWarps;
+    k_encode_rc<<<blocks < sms * 16 ? blocks : sms * 16, kRcWarps * 32, 0, s>>>(p, lanes);
     return cudaGetLastError();
 }
 
-cudaError_t launch_fracmap(const BlobParams &p, cudaStream_t s) {
+cudaError_t launch_fracmap(const EncParams &e, const BlobParams &p, cudaStream_t s) {
     if (p.nchunks <= 0) return cudaSuccess;
+    k_frac_count<<<(unsigned)((e.n + 7) / 8), 256, 0, s>>>(e);
+    const cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) return err;
     k_fracmap<<<p.nchunks, 32, 0, s>>>(p);
     return cudaGetLastError();
 }

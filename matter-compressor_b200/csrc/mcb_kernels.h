@@ -163,15 +163,15 @@ struct EncParams {
     uint32_t *len;       // per item: payload bytes (0 = all air, not coded)
     uint8_t *frac;       // per item: material nibble
     uint32_t *status;    // [0]: payloads that overflowed kEncCap
-    // symbol scratch between the transform and the coder, per item: levels in
-    // scan order (kN3 int16), corrections (kN3 u32: pos | delta << 16), and
-    // (coded flag | eob << 8 | dc, ncorr)
-    int16_t *levels;
+    // symbol scratch between the transform and the coder, per item: nonzero
+    // levels in scan order (kN3 u32: position | level << 16), corrections (kN3
+    // u32: pos | delta << 16), and (coded flag | eob << 8 | dc, ncorr)
+    uint32_t *entries;
     uint32_t *corr;
     uint2 *sym;
 };
-cudaError_t upload_cos_encode(const float cmf[16][16], cudaStream_t s);
-cudaError_t launch_encode(const EncParams &p, cudaStream_t s);      // transform: levels, corrections, nibbles
+cudaError_t upload_encode_tables(const float cmf[16][16], const uint16_t scan[kN3], cudaStream_t s);
+cudaError_t launch_encode(const EncParams &p, cudaStream_t s);      // transform: entries, corrections
 cudaError_t launch_encode_rc(const EncParams &p, cudaStream_t s);   // range coder, after it
 
 // Chunk-blob assembly for chunks whose blocks were encoded by launch_encode
@@ -194,7 +194,7 @@ struct BlobParams {
     uint8_t *blobs;
     uint64_t *hash;           // per chunk: the blob's chained xxh64 (the header's field stays 0)
 };
-cudaError_t launch_fracmap(const BlobParams &p, cudaStream_t s);       // fraction maps, after the transform
+cudaError_t launch_fracmap(const EncParams &e, const BlobParams &p, cudaStream_t s);   // nibbles and fraction maps
 cudaError_t launch_blob_layout(const BlobParams &p, cudaStream_t s);   // sizing pass, after both coders
 cudaError_t launch_blob_fill(const BlobParams &p, cudaStream_t s);     // write pass
 cudaError_t launch_blob_hash(const BlobParams &p, cudaStream_t s);     // xxh64 chain

@@ -91,7 +91,7 @@ static void runtime_init() {
     if (cudaMalloc(&R->d_scan, sizeof R->h_scan) != cudaSuccess ||
         cudaMalloc(&R->d_qtab, sizeof(QTab) * kMaxQSlots) != cudaSuccess ||
         cudaMemcpy(R->d_scan, R->h_scan, sizeof R->h_scan, cudaMemcpyHostToDevice) != cudaSuccess ||
-        upload_decode_tables(R->h_cos, R->h_scan, 0) != cudaSuccess || upload_cos_encode(R->h_cos, 0) != cudaSuccess ||
+        upload_decode_tables(R->h_cos, R->h_scan, 0) != cudaSuccess || upload_encode_tables(R->h_cos, R->h_scan, 0) != cudaSuccess ||
         preload_decode_kernels() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
         g_rt_err = std::string("device table upload failed: ") + cudaGetErrorString(cudaGetLastError());
         delete R;
@@ -639,7 +639,7 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
         !L.b_fml.ensure(4 * nchunks) || !L.b_np.ensure(4 * nchunks) || !L.b_len.ensure(8 * nchunks) ||
         !L.b_off.ensure(8 * nchunks) || !L.b_q.ensure(4 * nchunks) || !L.h_misc.ensure(24 * (size_t)nchunks) ||
         !L.b_hash.ensure(8 * (size_t)nchunks) || !encode_streams(L) ||
-        !L.enc_lv.ensure(2 * (size_t)kN3 * n) || !L.enc_corr.ensure(4 * (size_t)kN3 * n) || !L.enc_sym.ensure(8 * n))
+        !L.enc_ent.ensure(4 * (size_t)kN3 * n) || !L.enc_corr.ensure(4 * (size_t)kN3 * n) || !L.enc_sym.ensure(8 * n))
         return false;
     EncItem *hi = L.h_items.as<EncItem>();
     for (int c = 0; c < nchunks; ++c) {
@@ -671,7 +671,7 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
     ep.len = L.enc_len.as<uint32_t>();
     ep.frac = L.enc_frac.as<uint8_t>();
     ep.status = L.status.as<uint32_t>();
-    ep.levels = L.enc_lv.as<int16_t>();
+    ep.entries = L.enc_ent.as<uint32_t>();
     ep.corr = L.enc_corr.as<uint32_t>();
     ep.sym = L.enc_sym.as<uint2>();
     BlobParams bp;
@@ -690,16 +690,19 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
     bp.blob_off = L.b_off.as<uint64_t>();
     bp.blobs = nullptr;
     bp.hash = L.b_hash.as<uint64_t>();
-    // the fraction maps need the transform only: beside the block coder
-    if (!cuda_ok(launch_encode(ep, L.stream), "encode launch") ||
-        !cuda_ok(cudaEventRecord(L.ev_main, L.stream), "event record") ||
+    // the fraction maps need the voxels only: beside the transform and the block coder
+    if (!cuda_ok(cudaEventRecord(L.ev_main, L.stream), "event record") ||
         !cuda_ok(cudaStreamWaitEvent(L.side, L.ev_main, 0), "stream wait") ||
-        !cuda_ok(launch_fracmap(bp, L.side), "fraction map launch") ||
+        !cuda_ok(launch_fracmap(ep, bp, L.side), "fraction map launch") ||
         !cuda_ok(cudaEventRecord(L.ev_side, L.side), "event record") ||
+        !cuda_ok(launch_encode(ep, L.stream), "encode launch") ||
         !cuda_ok(launch_encode_rc(ep, L.stream), "range coder launch") ||
         !cuda_ok(cudaStreamWaitEvent(L.stream, L.ev_side, 0), "stream wait") ||
-        !cuda_ok(launch_blob_layout(bp, L.stream), "blob layout launch"))
+        !cuda_ok(launch_blob_layout(bp, L.stream), "blob layout launch")) {
+        cudaStreamSynchronize(L.side);   // nothing of this call outlives it
+        cudaStreamSynchronize(L.stream);
         return false;
+    }
     uint64_t *hl = reinterpret_cast<uint64_t *>(L.h_misc.as<uint8_t>() + 8 * (size_t)nchunks);
     uint32_t status = 0;
     if (!cuda_ok(cudaMemcpyAsync(hl, L.b_len.p, 8 * (size_t)nchunks, cudaMemcpyDeviceToHost, L.stream), "D2H") ||
