@@ -83,6 +83,13 @@ struct FusedParams {
 };
 int fused_grid(const LaunchCfg &cfg);   // CTAs of k_decode_fused (0: cannot launch)
 cudaError_t launch_fused(const FusedParams &f, const LaunchCfg &cfg, cudaStream_t s);
+// Arena offsets (base[i], entry_cap(len) entries each) and processing order
+// (longest payload first, absent blocks last) of n work items, on the device.
+// d_ws: kLayoutWords words.
+constexpr int kLayoutClasses = 1024;
+constexpr size_t kLayoutWords = 2 * kLayoutClasses + 2;   // counts, places taken, the arena's 64-bit total
+cudaError_t launch_layout(const DecItem *d_items, int n, uint64_t *d_base, uint32_t *d_order, uint32_t *d_ws,
+                          cudaStream_t s);
 // The decode kernels' constant tables: the cosine basis and the band ends of
 // the scan order (scan position -> raster idx | band << 12).
 cudaError_t upload_decode_tables(const float cmf[16][16], const uint16_t scan[kN3], cudaStream_t s);

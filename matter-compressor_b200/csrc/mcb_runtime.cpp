@@ -436,10 +436,26 @@ bool decode_prepare_staged(DecodeBatch &B, int n, cudaStream_t s) {
     B.n = n;
     B.subs.clear();
     if (n <= 0) return true;
+    const DecItem *items = B.h_items.as<DecItem>();
+    uint64_t acc = 0;
+    int coded = 0;
+    for (int i = 0; i < n; ++i) {
+        acc += entry_cap(items[i].len);
+        coded += items[i].len > 0;
+    }
+    if (acc <= kArenaMaxEntries) {
+        B.subs.emplace_back(0, n);
+        B.coded.assign(1, coded);
+        B.split.assign(1, 0);
+        return batch_buffers(B, n, acc) && B.lws.ensure(sizeof(uint32_t) * kLayoutWords) &&
+               cuda_ok(cudaMemcpyAsync(B.items.p, items, sizeof(DecItem) * (size_t)n, cudaMemcpyHostToDevice, s),
+                       "H2D items") &&
+               cuda_ok(launch_layout(B.items.as<DecItem>(), n, B.base.as<uint64_t>(), B.order.as<uint32_t>(),
+                                     B.lws.as<uint32_t>(), s), "layout launch");
+    }
     if (!B.h_order.ensure(sizeof(uint32_t) * (size_t)n) || !B.h_base.ensure(sizeof(uint64_t) * (size_t)n) ||
         !B.h_rec.ensure(sizeof(uint32_t) * (size_t)n))
         return false;
-    const DecItem *items = B.h_items.as<DecItem>();
     const uint64_t max_acc =
         batch_layout(B, items, n, B.h_base.as<uint64_t>(), B.h_order.as<uint32_t>(), B.h_rec.as<uint32_t>());
     return batch_buffers(B, n, max_acc) &&

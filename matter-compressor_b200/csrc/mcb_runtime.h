@@ -66,6 +66,7 @@ float slot_quality(int slot);
 struct DecodeBatch {
     DevBuf items, order, base, hdr, arena, pool, status, rec_idx;
     DevBuf fws;   // work area of the fused decode kernel
+    DevBuf lws;   // work area of the device layout
     HostBuf h_items, h_order, h_base, h_status, h_rec;   // pinned staging of decode_prepare_staged
     int n = 0;
     std::vector<std::pair<int, int>> subs;   // [i0, i1) ranges that fit the arena
@@ -122,9 +123,11 @@ Lane *lane();
 
 bool decode_prepare(DecodeBatch &B, const DecItem *h_items, int n, cudaStream_t s);
 // decode_prepare without any host synchronisation: the n items are already in
-// B.h_items (pinned), order and offsets are built in B's pinned staging, and
-// every upload is asynchronous on s. The caller guarantees that the batch's
-// previous use has completed.
+// B.h_items (pinned) and are uploaded asynchronously on s, where order and
+// offsets are then made by the device (mcb_layout.cu); a batch beyond one
+// arena is laid out in sub-batches in B's pinned staging instead. No split-off
+// long blocks (DecodeBatch::split) either way: that is a plan's layout. The
+// caller guarantees that the batch's previous use has completed.
 bool decode_prepare_staged(DecodeBatch &B, int n, cudaStream_t s);
 // Creates the stream and event of a pipeline slot on first use.
 bool blob_slot_ready(BlobSlot &S);
