@@ -580,14 +580,13 @@ int mc_b200_decode_chunk_blobs(const uint8_t *const *blobs, const uint64_t *lens
                                              S.stream), "H2D blob") &&
                      blob_items(b, lens[c0 + j], S.src.as<uint8_t>() + at[j], it);
         }
-        // groups decode while others are in flight, so the lane-per-block
-        // kernel's fewer instructions per bin count, not one group's chain
-        // length: no single-thread share (measured on 64 chunks: 49.0 GB/s
-        // against 45.5 with the share by block count, 43.7 with it for the
-        // first group only, whose single-thread kernel holds every SM's
-        // registers while the next group waits to start)
+        // groups decode while others are in flight, so the lane kernel's fewer
+        // instructions per bin count, but for the few longest blocks, whose chains
+        // hold the group's copy-out back (64 chunks at q=6 20.23 ms with lanes
+        // alone, 20.13 so, 20.56 with every block on a single thread; 16 chunks at
+        // q=1 10.17, 9.93, 15.85; 3 chunks at q=6 1.79, 1.65, 1.61)
         LaunchCfg cfg = L->cfg;
-        if (cfg.ent_solo < 0) cfg.ent_solo = 0;
+        if (cfg.ent_solo < 0) cfg.ent_solo = 32;
         ok = ok && decode_prepare_staged(B, (int)ni, S.stream) && decode_enqueue(B, cfg, S.stream) &&
              cuda_ok(cudaMemcpyAsync(B.h_status.p, B.status.p, 4, cudaMemcpyDeviceToHost, S.stream), "D2H status");
         if (!ok) break;

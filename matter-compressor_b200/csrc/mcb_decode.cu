@@ -569,32 +569,37 @@ __device__ __forceinline__ void run_lanes(LaneState &L, const EntParams &P, uint
 
 // The whole stream of one block on one thread, after lane_begin, written for
 // the latency of one thread alone on its warp (no other lane shares its
-// instructions). All contexts of the coefficient loop that the common bins
-// use are held in registers: the four significance contexts of the current
-// band and the twelve magnitude rungs. Bands only advance, so a band's
-// register contexts are never written back to shared memory, and the magnitude
-// rungs are used by nothing else. The common steps use selects rather than
-// branches, whose divergence bookkeeping costs more than their work.
-// Two loops take the significance bins. Where three or more of the last 16
-// positions were significant (density class 3), half of the positions are, and
-// the loop takes one bin at a time, its probability in the class's own
-// register. In the sparser classes runs of zeros are long and go four at a
-// time: while bins are 0 the code does not change and the range only falls, so
-// four splits are computed straight through and one compare of the last with
-// the code and the renormalisation bound decides them all.
-// Band changes and the corrections take the shared step functions
-// (position_event, put_entry, slow_work).
+// instructions). What bounds it: the chain of dependent instructions (five
+// cycles each) and the branches, a third of the cycles. So every decision jumps
+// straight to where the next bin is decoded: with the same work in nested loops
+// whose flags were tested again at each level it took a fifth longer (48 blocks
+// at q=6: 5.76 against 4.66 ms), and a renormalisation decided by a branch, not
+// by selects, took another 4 % off (4.50; 5.94 before runs of zeros).
+// All contexts of the coefficient loop that the common bins use are held in
+// registers: the four significance contexts of the current band and the twelve
+// magnitude rungs. Bands only advance, so a band's register contexts are never
+// written back to shared memory, and the magnitude rungs are used by nothing
+// else.
+// Where three or more of the last 16 positions were significant (density class
+// 3), half of the positions are, and bins go one at a time, their probability in
+// the class's own register. In the sparser classes runs of zeros are long and go
+// four at a time: while bins are 0 the code does not change and the range only
+// falls, so four splits are computed straight through and one compare of the
+// last with the code and the renormalisation bound decides them all.
+// Band changes, Exp-Golomb tails and the corrections take the shared functions
+// (position_event, eg_value, put_entry, slow_work).
 
-// Renormalisation with the common case (one byte) by selects; a second byte
-// or a window refill takes the loop.
-__device__ __forceinline__ void renorm_sel(LaneState &L) {
-    const uint32_t s = L.range < kTop ? 8u : 0u;
-    L.code = funnel_left(L.w << L.used, L.code, s);
-    L.range <<= s;
-    L.used += s;
-    if ((L.used == 32u) | (L.range < kTop)) {
-        if (L.used == 32u) refill(L);
-        renorm(L);
+// The window while the thread is alone: w shifted to its next byte, `used` bits
+// gone from it; shifted back for the shared functions that read bytes.
+__device__ __forceinline__ void window_in(LaneState &L) { L.w <<= L.used; }
+__device__ __forceinline__ void window_out(LaneState &L) { L.w >>= L.used; }
+__device__ __forceinline__ void solo_norm(LaneState &L) {
+    while (L.range < kTop) {
+        L.code = funnel_left(L.w, L.code, 8);
+        L.w <<= 8;
+        L.range <<= 8;
+        L.used += 8;
+        if (L.used == 32) refill(L);
     }
 }
 // One adaptive bin on a register context.
@@ -604,7 +609,7 @@ __device__ __forceinline__ bool reg_bin(LaneState &L, uint32_t &g) {
     L.code = b ? L.code - r : L.code;
     L.range = b ? L.range - r : r;
     g = (15u * g + (b ? 15u : 4096u)) >> 4;
-    renorm_sel(L);
+    solo_norm(L);
     return b;
 }
 // One magnitude rung on a register context; after a 1 the range is
@@ -619,7 +624,7 @@ __device__ __forceinline__ bool rung(LaneState &L, uint32_t &g) {
     L.code -= r;
     L.range -= r;
     g = prob_after1(g);
-    if (L.range < kTop) renorm(L);
+    solo_norm(L);
     return true;
 }
 // One bypass bin (src/mc_codec.c:205).
@@ -627,7 +632,7 @@ __device__ __forceinline__ bool reg_bypass(LaneState &L) {
     L.range >>= 1;
     const bool b = L.code >= L.range;
     L.code = b ? L.code - L.range : L.code;
-    renorm_sel(L);
+    solo_norm(L);
     return b;
 }
 
@@ -640,101 +645,115 @@ __device__ __forceinline__ void solo_entropy(LaneState &L, const EntParams &P, u
     uint32_t g3 = ctx[(kCtxMag + 3) * 32], g4 = ctx[(kCtxMag + 4) * 32], g5 = ctx[(kCtxMag + 5) * 32];
     uint32_t g6 = ctx[(kCtxMag + 6) * 32], g7 = ctx[(kCtxMag + 7) * 32], g8 = ctx[(kCtxMag + 8) * 32];
     uint32_t g9 = ctx[(kCtxMag + 9) * 32], g10 = ctx[(kCtxMag + 10) * 32], g11 = ctx[(kCtxMag + 11) * 32];
-    bool one = L.st == S_LAST;   // the position at p - 1 is significant, its coefficient is next
-    bool more = L.st <= S_LAST;
-    while (more) {
-        if (!one) {
-            if (L.p < L.e3) {   // density class 3
-                const uint32_t end = min(L.stop, L.e3);
-                for (;;) {
-                    const uint32_t r = (L.range >> 12) * s3;
-                    if (L.code >= r) {   // significant
-                        L.code -= r;
-                        L.range -= r;
-                        s3 = prob_after1(s3);
-                        ++L.p;
-                        renorm_sel(L);
-                        one = true;
-                        break;
-                    }
-                    L.range = r;
-                    s3 = prob_after0(s3);
-                    ++L.p;
-                    if ((r < kTop) | (L.p >= end)) {
-                        if (r < kTop) renorm(L);
-                        if (L.p >= end) break;
-                    }
-                }
-            } else {
-                const bool a2 = L.p < L.e2, a1 = L.p < L.e1;
-                const uint32_t end = min(L.stop, a2 ? L.e2 : (a1 ? L.e1 : 0xFFFFFFFFu));
-                uint32_t pc = a2 ? s2 : (a1 ? s1 : s0);
-                do {
-                    const uint32_t floor1 = L.code >= kTop ? L.code : kTop - 1u;
-                    while (L.p + 4u <= end) {
-                        const uint32_t r1 = (L.range >> 12) * pc, q1 = prob_after0(pc);
-                        const uint32_t r2 = (r1 >> 12) * q1, q2 = prob_after0(q1);
-                        const uint32_t r3 = (r2 >> 12) * q2, q3 = prob_after0(q2);
-                        const uint32_t r4 = (r3 >> 12) * q3;
-                        if (r4 <= floor1) break;
-                        L.range = r4;
-                        pc = prob_after0(q3);
-                        L.p += 4;
-                    }
-                    if (L.p >= end) break;
-                    one = reg_bin(L, pc);
-                    ++L.p;
-                } while (!one & (L.p < end));
+    uint32_t pc, m;
+    window_in(L);
+    if (L.st == S_LAST) goto coef;   // the implicit last position is all there is
+    if (L.st != F_RUN) goto done;
+next:   // a significance bin at p < stop
+    if (L.p < L.e3) {   // density class 3
+        const uint32_t r = (L.range >> 12) * s3;
+        ++L.p;
+        if (L.code >= r) {   // significant
+            L.code -= r;
+            L.range -= r;
+            s3 = prob_after1(s3);
+            solo_norm(L);
+            goto one;
+        }
+        L.range = r;
+        s3 = prob_after0(s3);
+        if ((r < kTop) | (L.p >= L.stop)) {
+            solo_norm(L);
+            if (L.p >= L.stop) goto position;
+        }
+        goto next;
+    } else {
+        const bool a2 = L.p < L.e2, a1 = L.p < L.e1;
+        const uint32_t end = min(L.stop, a2 ? L.e2 : (a1 ? L.e1 : 0xFFFFFFFFu));
+        pc = a2 ? s2 : (a1 ? s1 : s0);
+    run:
+        {
+            const uint32_t floor1 = L.code >= kTop ? L.code : kTop - 1u;
+            while (L.p + 4u <= end) {
+                const uint32_t r1 = (L.range >> 12) * pc, q1 = prob_after0(pc);
+                const uint32_t r2 = (r1 >> 12) * q1, q2 = prob_after0(q1);
+                const uint32_t r3 = (r2 >> 12) * q2, q3 = prob_after0(q2);
+                const uint32_t r4 = (r3 >> 12) * q3;
+                if (r4 <= floor1) break;
+                L.range = r4;
+                pc = prob_after0(q3);
+                L.p += 4;
+            }
+        }
+        if (L.p < end) {
+            const uint32_t r = (L.range >> 12) * pc;
+            ++L.p;
+            if (L.code >= r) {
+                L.code -= r;
+                L.range -= r;
+                pc = prob_after1(pc);
+                solo_norm(L);
                 s0 = a1 ? s0 : pc;
                 s1 = a1 & !a2 ? pc : s1;
                 s2 = a2 ? pc : s2;
+                goto one;
             }
-            if (one) {
-                L.e3 = L.e2;
-                L.e2 = L.e1;
-                L.e1 = L.p + 16u;
-            }
+            L.range = r;
+            pc = prob_after0(pc);
+            solo_norm(L);
+            if (L.p < end) goto run;
         }
-        if (one) {
-            // the coefficient at p - 1: the unary magnitude
-            // (src/mc_codec.c:268-275), the sign, the entry
-            uint32_t m = 1;
-            if (reg_bin(L, g0)) {
-                if (!rung(L, g1)) m = 2;
-                else if (!rung(L, g2)) m = 3;
-                else if (!rung(L, g3)) m = 4;
-                else if (!rung(L, g4)) m = 5;
-                else if (!rung(L, g5)) m = 6;
-                else if (!rung(L, g6)) m = 7;
-                else if (!rung(L, g7)) m = 8;
-                else if (!rung(L, g8)) m = 9;
-                else if (!rung(L, g9)) m = 10;
-                else if (!rung(L, g10)) m = 11;
-                else if (!rung(L, g11)) m = 12;
-                else {   // the twelfth rung set: 12 + an Exp-Golomb value
-                    m = 12u + eg_value(L);
-                    if (L.bad) { L.st = S_DONE; break; }   // prefix cap (corrupt streams only)
-                }
-                renorm(L);
-            }
-            const bool neg = reg_bypass(L);
-            const uint32_t v = (L.p - 1u) | ((neg ? 0u - m : m) << 16);
-            if (L.nent < L.cap) L.ent[L.nent++] = v;
-            else if (!put_entry(L, P, v)) break;   // overflow pool exhausted (corrupt streams only)
-            L.st = F_RUN;
-            one = false;
-        }
-        if (L.p >= L.stop) {   // the band's contexts come into registers when it changes
-            position_event(L, ctx, s_bend);
-            if (L.sigb != sigb) {
-                sigb = L.sigb;
-                s0 = ctx[(sigb + 0) * 32]; s1 = ctx[(sigb + 1) * 32];
-                s2 = ctx[(sigb + 2) * 32]; s3 = ctx[(sigb + 3) * 32];
-            }
-            one = L.st == S_LAST;
-            more = L.st <= S_LAST;
+        s0 = a1 ? s0 : pc;
+        s1 = a1 & !a2 ? pc : s1;
+        s2 = a2 ? pc : s2;
+        if (L.p >= L.stop) goto position;
+        goto next;
+    }
+one:
+    L.e3 = L.e2;
+    L.e2 = L.e1;
+    L.e1 = L.p + 16u;
+coef:   // the coefficient at p - 1: the unary magnitude (src/mc_codec.c:268-275), the sign, the entry
+    m = 1;
+    if (rung(L, g0)) {
+        if (!rung(L, g1)) m = 2;
+        else if (!rung(L, g2)) m = 3;
+        else if (!rung(L, g3)) m = 4;
+        else if (!rung(L, g4)) m = 5;
+        else if (!rung(L, g5)) m = 6;
+        else if (!rung(L, g6)) m = 7;
+        else if (!rung(L, g7)) m = 8;
+        else if (!rung(L, g8)) m = 9;
+        else if (!rung(L, g9)) m = 10;
+        else if (!rung(L, g10)) m = 11;
+        else if (!rung(L, g11)) m = 12;
+        else {   // the twelfth rung set: 12 + an Exp-Golomb value
+            window_out(L);
+            m = 12u + eg_value(L);
+            window_in(L);
+            if (L.bad) { L.st = S_DONE; goto done; }   // prefix cap (corrupt streams only)
         }
     }
+    solo_norm(L);
+    {
+        const bool neg = reg_bypass(L);
+        const uint32_t v = (L.p - 1u) | ((neg ? 0u - m : m) << 16);
+        if (L.nent < L.cap) L.ent[L.nent++] = v;
+        else if (!put_entry(L, P, v)) goto done;   // overflow pool exhausted (corrupt streams only)
+    }
+    if (L.p < L.stop) goto next;
+position:
+    L.st = F_RUN;
+    position_event(L, ctx, s_bend);
+    if (L.sigb != sigb) {   // the band's contexts come into registers when it changes
+        sigb = L.sigb;
+        s0 = ctx[(sigb + 0) * 32]; s1 = ctx[(sigb + 1) * 32];
+        s2 = ctx[(sigb + 2) * 32]; s3 = ctx[(sigb + 3) * 32];
+    }
+    if (L.st == F_RUN) goto next;
+    if (L.st == S_LAST) goto coef;
+done:
+    window_out(L);
     while (L.st != S_DONE) slow_work(L, P, ctx, s_bend);
 }
 
@@ -1863,14 +1882,14 @@ static cudaError_t launch_entropy_w(const EntParams &p, int ctas_per_sm, cudaStr
 }
 
 // The single-thread share when a launch configuration leaves it open, from
-// the launch's coded blocks. Below about 4 chunks' worth the stage's time is the
-// longest block's chain, which a single thread runs fastest (q=6: 2 chunks 530
-// us against 723 with lanes alone, 4 chunks 584 against 745; q=12: 281 against
-// 391). Up to about 60 chunks' worth the longest blocks, four for each SM (one
+// the launch's coded blocks. Below about 5 chunks' worth the stage's time is the
+// longest block's chain, which a single thread runs fastest (q=6: 2 chunks 352
+// us against 723 with lanes alone, 4 chunks 461 against 745; q=12: 244 against
+// 399). Up to about 60 chunks' worth the longest blocks, four for each SM (one
 // for each of its schedulers), run on single threads beside the lanes (8 chunks
-// 643 us against 764 with lanes alone and 1042 on single threads; 16: 762 / 848
-// / 2087; 48: 1250 / 1333); a full 64 chunks gain nothing (1548 / 1554).
-constexpr int kSoloAllMax = 15 * 1024, kSoloShareMax = 200 * 1024;
+// 637 us against 770 with lanes alone and 791 on single threads; 16: 745 / 850
+// / 1583; 32: 940 / 1055); a full 64 chunks gain nothing (1.55 ms).
+constexpr int kSoloAllMax = 19 * 1024, kSoloShareMax = 200 * 1024;
 static int auto_solo(int ncoded) {
     if (ncoded <= kSoloAllMax) return 1;
     return ncoded <= kSoloShareMax ? ncoded / (4 * num_sms()) : 0;
