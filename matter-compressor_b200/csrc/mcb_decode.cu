@@ -758,7 +758,7 @@ done:
 }
 
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) k_entropy(EntParams P) {
+__global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_entropy(EntParams P) {
     // s_bend[b]: first scan position past band b; then the lanes' contexts,
     // context j of lane l of warp w at word (w * kCtxSlots + j) * 32 + l
     extern __shared__ uint32_t s_ent[];
