@@ -961,6 +961,27 @@ cudaError_t upload_encode_tables(const float cmf[16][16], const uint16_t scan[kN
     return e != cudaSuccess ? e : cudaMemcpyToSymbolAsync(c_bend, bend, sizeof bend, 0, cudaMemcpyHostToDevice, s);
 }
 
+// The items of whole chunks, block by block: made where they are read, instead
+// of 1.3 MB for 8 chunks built and uploaded by the host (0.2 ms of a call).
+__global__ void __launch_bounds__(256) k_encode_items(EncChunks c, EncItem *items, uint8_t *pay) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x, k = i >> 12, b = i & 4095u;
+    EncItem it;
+    it.src = (uint64_t)(uintptr_t)(c.vox[k] + (size_t)((b >> 8) * 16) * 65536 + ((b >> 4) & 15) * (16 * 256) + (b & 15) * 16);
+    it.sz = 65536;
+    it.sy = 256;
+    it.out = (uint64_t)(uintptr_t)(pay + (size_t)i * kEncCap);
+    it.qslot = c.qslot[k];
+    it.tau = c.tau[k];
+    it.pad = 0;
+    items[i] = it;
+}
+
+cudaError_t launch_encode_items(const EncChunks &c, EncItem *d_items, uint8_t *d_pay, cudaStream_t s) {
+    if (c.n <= 0) return cudaSuccess;
+    k_encode_items<<<c.n * (kGrid3 / 256), 256, 0, s>>>(c, d_items, d_pay);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_encode(const EncParams &p, cudaStream_t s) {
     if (p.n <= 0) return cudaSuccess;
     const int smem = (int)sizeof(EncSmem);

@@ -178,6 +178,15 @@ struct EncParams {
     uint2 *sym;
 };
 cudaError_t upload_encode_tables(const float cmf[16][16], const uint16_t scan[kN3], cudaStream_t s);
+// Up to kEncChunks whole chunks of 256^3 voxels (c.vox[k], dense) as 4096 items
+// each, block by block, payload slots kEncCap bytes apart from d_pay on.
+constexpr int kEncChunks = 8;
+struct EncChunks {
+    const uint8_t *vox[kEncChunks];
+    uint16_t qslot[kEncChunks], tau[kEncChunks];
+    int n;
+};
+cudaError_t launch_encode_items(const EncChunks &c, EncItem *d_items, uint8_t *d_pay, cudaStream_t s);
 cudaError_t launch_encode(const EncParams &p, cudaStream_t s);      // transform: entries, corrections
 cudaError_t launch_encode_rc(const EncParams &p, cudaStream_t s);   // range coder, after it
 

@@ -648,7 +648,7 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
     if (nchunks <= 0) return true;
     if (!cuda_ok(cudaEventSynchronize(L.done), "event sync")) return false;
     const size_t n = (size_t)nchunks * kGrid3;
-    if (!L.h_items.ensure(sizeof(EncItem) * n) || !L.enc_items.ensure(sizeof(EncItem) * n) ||
+    if (!L.enc_items.ensure(sizeof(EncItem) * n) ||
         !L.enc_len.ensure(4 * n) || !L.enc_frac.ensure(n) || !L.enc_pay.ensure((size_t)kEncCap * n) ||
         !L.status.ensure(16) || !L.b_scratch.ensure(4 * n) || !L.b_lens16.ensure(2 * n) ||
         !L.b_bitmap.ensure((size_t)kBitmapBytes * nchunks) || !L.b_fmap.ensure((size_t)kFmapCap * nchunks) ||
@@ -657,26 +657,24 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
         !L.b_hash.ensure(8 * (size_t)nchunks) || !encode_streams(L) ||
         !L.enc_ent.ensure(4 * (size_t)kN3 * n) || !L.enc_corr.ensure(4 * (size_t)kN3 * n) || !L.enc_sym.ensure(8 * n))
         return false;
-    EncItem *hi = L.h_items.as<EncItem>();
-    for (int c = 0; c < nchunks; ++c) {
-        int slot = qslot(q[c]);
-        if (slot < 0) return false;
-        for (int bi = 0; bi < kGrid3; ++bi) {
-            int bz = bi >> 8, by = (bi >> 4) & 15, bx = bi & 15;
-            EncItem &it = hi[(size_t)c * kGrid3 + bi];
-            it.src = (uint64_t)(uintptr_t)(d_vox[c] + (size_t)(bz * 16) * 65536 + (by * 16) * 256 + bx * 16);
-            it.sz = 65536;
-            it.sy = 256;
-            it.out = (uint64_t)(uintptr_t)(L.enc_pay.as<uint8_t>() + ((size_t)c * kGrid3 + bi) * kEncCap);
-            it.qslot = (uint16_t)slot;
-            it.tau = (uint16_t)std::min(std::max(tau[c], 0), 65535);
-            it.pad = 0;
+    for (int c0 = 0; c0 < nchunks; c0 += kEncChunks) {
+        EncChunks ec;
+        ec.n = std::min(kEncChunks, nchunks - c0);
+        for (int j = 0; j < ec.n; ++j) {
+            const int slot = qslot(q[c0 + j]);
+            if (slot < 0) return false;
+            ec.vox[j] = d_vox[c0 + j];
+            ec.qslot[j] = (uint16_t)slot;
+            ec.tau[j] = (uint16_t)std::min(std::max(tau[c0 + j], 0), 65535);
         }
+        if (!cuda_ok(launch_encode_items(ec, L.enc_items.as<EncItem>() + (size_t)c0 * kGrid3,
+                                         L.enc_pay.as<uint8_t>() + (size_t)c0 * kGrid3 * kEncCap, L.stream),
+                     "encode items launch"))
+            return false;
     }
     float *hq = L.h_misc.as<float>();
     memcpy(hq, header_q, 4 * (size_t)nchunks);
-    if (!cuda_ok(cudaMemcpyAsync(L.enc_items.p, hi, sizeof(EncItem) * n, cudaMemcpyHostToDevice, L.stream), "H2D") ||
-        !cuda_ok(cudaMemcpyAsync(L.b_q.p, hq, 4 * (size_t)nchunks, cudaMemcpyHostToDevice, L.stream), "H2D") ||
+    if (!cuda_ok(cudaMemcpyAsync(L.b_q.p, hq, 4 * (size_t)nchunks, cudaMemcpyHostToDevice, L.stream), "H2D") ||
         !cuda_ok(cudaMemsetAsync(L.status.p, 0, 16, L.stream), "memset"))
         return false;
     EncParams ep;
