@@ -905,9 +905,7 @@ int mc_b200_append_chunks(mc_archive *a, mc_codec_ctx *C, int lod, const int *co
                 dv[j] = vox[c0 + j];
             } else {
                 dv[j] = L->src.as<uint8_t>() + kChunkBytes * j;
-                if (!cuda_ok(cudaMemcpyAsync(const_cast<uint8_t *>(dv[j]), vox[c0 + j], kChunkBytes,
-                                             cudaMemcpyHostToDevice, L->stream), "H2D voxels"))
-                    return -1;
+                if (!copy_to_device(*L, const_cast<uint8_t *>(dv[j]), vox[c0 + j], kChunkBytes)) return -1;
             }
             if (C) {   // caller's context: its quality and max error (src/mc_archive.c:590-601)
                 hq[j] = qq[j] = C->quality;

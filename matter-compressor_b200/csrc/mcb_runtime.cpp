@@ -293,7 +293,11 @@ bool copy_to_host(Lane &L, uint8_t *dst, const uint8_t *d_src, size_t n, size_t 
 
 bool copy_to_device(Lane &L, uint8_t *d_dst, const uint8_t *src, size_t n) {
     constexpr size_t kPiece = 8u << 20;
-    if (n <= kPiece)
+    // pinned: one copy at the link's rate; a small pageable one too
+    cudaPointerAttributes pa;
+    const bool pageable = cudaPointerGetAttributes(&pa, src) != cudaSuccess || pa.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();   // a pageable pointer may leave an error behind on older drivers
+    if (!pageable || n <= kPiece)
         return cuda_ok(cudaMemcpyAsync(d_dst, src, n, cudaMemcpyHostToDevice, L.stream), "H2D");
     constexpr int K = 3;
     for (int k = 0; k < K; ++k)

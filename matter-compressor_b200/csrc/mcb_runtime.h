@@ -144,7 +144,7 @@ bool decode_enqueue_stage(DecodeBatch &B, const LaunchCfg &cfg, int stage, cudaS
 // segment k bound for dst + k * dst_stride.
 bool copy_to_host(Lane &L, uint8_t *dst, const uint8_t *d_src, size_t n, size_t seg = 0, size_t dst_stride = 0);
 // The other direction, for large ranges of pageable host memory (a mapped
-// archive file): host threads fill 8 MiB pinned pieces while earlier pieces
+// archive file, a caller's voxels): host threads fill 8 MiB pinned pieces while earlier pieces
 // cross the link. The copies are enqueued on the lane's stream; the call
 // returns once the last piece has been handed to the stream, so later work
 // on the stream sees the bytes. False on a CUDA error.
