@@ -27,6 +27,7 @@
 #include <stdint.h>
 
 #include "mcb_devinfo.h"
+#include "mcb_f32x2.cuh"
 #include "mcb_format.h"
 #include "mcb_kernels.h"
 #include "mcb_rowstore.cuh"
@@ -790,14 +791,14 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_entropy(EntParams P)
 constexpr size_t entropy_smem(int warps) { return 32 + sizeof(uint32_t) * kCtxSlots * 32 * (size_t)warps; }
 
 // The entropy stage with every block on a single thread: each warp's first
-// thread decodes blocks of the order one after another (entry `warp` first,
-// then claims from the counter), the other 31 threads leave at once. Entries go
-// to the CTAs in turn, and the second half of the CTAs starts at its third
-// warp, so that a small batch spreads over all SMs and their schedulers (the
-// stage at q=6: 1 chunk 393 us, 2 chunks 459; with entries 0..15 on the first
-// CTA and so on, 454 and 530). A block
-// then costs a few times fewer cycles per bin than as a lane of k_entropy, at
-// several times the issue slots per bin, which pays where a batch is too
+// thread decodes blocks of the order one after another (its own entry first,
+// then claims from the counter), the other 31 threads leave at once. First
+// entries go to the CTAs in turn, and the second half of the CTAs starts at its
+// third warp, so that a small batch spreads over all SMs and their schedulers
+// (with entries 0..15 on the first CTA and so on, the stage at q=6 took 16 %
+// longer at 1 chunk and 15 % at 2). A block then costs a few times fewer cycles
+// per bin than as a lane of k_entropy, at several times the issue slots per bin,
+// which pays where a batch is too
 // small to fill the machine and its longest blocks set the stage's time. The
 // threads' contexts share one 32-column region of shared memory (column =
 // warp index), conflict-free like k_entropy's. Two CTAs of 16 warps per SM
@@ -827,37 +828,7 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
 
-// Packed pairs: sm_100 executes two IEEE single-precision round-to-nearest
-// adds or multiplies per instruction (add/sub/mul.rn.f32x2), each lane of the
-// pair rounding exactly like its scalar __fadd_rn / __fmul_rn. One caution,
-// measured with ptxas 12.9 on sm_100a: a packed multiply whose result feeds a
-// packed add is contracted into a single-rounding packed FMA despite the .rn
-// qualifiers (even inside one asm statement, and also when the product is
-// written as fma with a -0 addend). The multiply-accumulates below therefore
-// pair a packed multiply with scalar __fadd_rn adds, a combination that keeps
-// both roundings; packed adds are used only on sums.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("{.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-        "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;}"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-    float2 d;
-    asm("{.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-        "sub.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;}"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("{.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-        "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;}"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-// acc + w*v per lane with two roundings (see above)
+// acc + w*v per lane with two roundings (see mcb_f32x2.cuh)
 __device__ __forceinline__ float2 madd2(float2 acc, float2 w, float2 v) {
     const float2 p = mul2(w, v);
     return make_float2(__fadd_rn(acc.x, p.x), __fadd_rn(acc.y, p.y));

@@ -18,14 +18,17 @@
 #include <stdint.h>
 
 #include "mcb_devinfo.h"
+#include "mcb_f32x2.cuh"
 #include "mcb_format.h"
 #include "mcb_kernels.h"
 
 namespace mcb {
 
-// this translation unit's copies (no -rdc): the cosine basis, and the first scan
-// position past each band (b < 7), then kN3 and a sentinel
-__constant__ float c_cos[16][16];
+// this translation unit's copies (no -rdc): the cosine basis c[k][n] with every
+// value doubled, as [n][k] and as [k][n] for n < 8, and the first scan position past
+// each band (b < 7), then kN3 and a sentinel
+__constant__ float4 c_fwd[8][8];
+__constant__ float4 c_inv[16][4];
 __constant__ uint16_t c_bend[9];
 
 namespace {
@@ -65,63 +68,106 @@ __device__ __forceinline__ void enc_norm(Enc &e) {
 }
 __device__ __forceinline__ int bitlen32(uint32_t v) { return v ? 32 - __clz(v) : 0; }
 // ------------------------------------------------------------ transforms
-// forward DCT-II, outputs k in {j, j+4, j+8, j+12} of one line
-__device__ __forceinline__ void fdct_quad(const float *in, int si, float *out, int so, int j) {
-    float s[8], d[8];
+// Two adjacent lines per thread, packed: value n of both lines is in[n * st].
+// Every sum runs over ascending n (forward) or k (inverse), as the reference's
+// (src/mc_codec_float.h:70-158). The adds take the products of the iteration
+// before, which reach them through the loop's back edge (see mcb_f32x2.cuh). A sum
+// starts from its first product, not from 0 plus it: only the sign of a zero can
+// differ, which no level and no voxel shows.
+__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+// forward DCT-II, all 16 outputs
+__device__ __forceinline__ void dct_products(float2 q[16], float2 a, float2 b, const float4 *w) {
+    const float2 s = add2(a, b), d = sub2(a, b);
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-        float a = in[n * si], b = in[(15 - n) * si];
-        s[n] = fadd(a, b);
-        d[n] = fsub(a, b);
-    }
-    const bool odd = j & 1;    // k = j + 4q keeps the parity of j
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        int k = j + 4 * q;
-        float acc = 0.0f;
-#pragma unroll
-        for (int n = 0; n < 8; ++n) acc = fadd(acc, fmul(c_cos[k][n], odd ? d[n] : s[n]));
-        out[k * so] = acc;
+    for (int k = 0; k < 8; ++k) {
+        q[2 * k] = mul2(lo2(w[k]), s);
+        q[2 * k + 1] = mul2(hi2(w[k]), d);
     }
 }
-// inverse DCT-III over all 16 k, outputs n and 15-n for n in {j, j+4}
-__device__ __forceinline__ void idct_quad(const float *in, int si, float *out, int so, int j) {
+__device__ __forceinline__ void dct_lines(const float2 *in, int st, float2 o[16]) {
+    const float2 *end = in + 15 * st;
+    const float4 *w = c_fwd[0];
+    float2 q[16];
+    dct_products(o, *in, *end, w);
+    in += st; end -= st; w += 8;
+    dct_products(q, *in, *end, w);
+#pragma unroll 1
+    for (int n = 2;; ++n) {
+        in += st; end -= st; w += 8;
+        const float2 a = *in, b = *end;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        int n = j + 4 * q;
-        float ev = 0.0f, od = 0.0f;
+        for (int k = 0; k < 16; ++k) o[k] = add2(o[k], q[k]);
+        dct_products(q, a, b, w);
+        if (n == 7) break;
+    }
 #pragma unroll
-        for (int k = 0; k < 16; k += 2) ev = fadd(ev, fmul(c_cos[k][n], in[k * si]));
+    for (int k = 0; k < 16; ++k) o[k] = add2(o[k], q[k]);
+}
+// inverse DCT-III, all 16 outputs from all 16 inputs
+__device__ __forceinline__ void idct_products(float2 q[16], float2 e, float2 o, const float4 *w) {
 #pragma unroll
-        for (int k = 1; k < 16; k += 2) od = fadd(od, fmul(c_cos[k][n], in[k * si]));
-        out[n * so] = fadd(ev, od);
-        out[(15 - n) * so] = fsub(ev, od);
+    for (int m = 0; m < 4; ++m) {
+        q[2 * m] = mul2(lo2(w[m]), e);
+        q[2 * m + 1] = mul2(hi2(w[m]), e);
+        q[8 + 2 * m] = mul2(lo2(w[4 + m]), o);
+        q[8 + 2 * m + 1] = mul2(hi2(w[4 + m]), o);
+    }
+}
+__device__ __forceinline__ void idct_lines(const float2 *in, int st, float2 o[16]) {
+    const float4 *w = c_inv[0];
+    float2 a[16], q[16];   // the even-k sums of outputs 0-7, then the odd-k ones
+    idct_products(a, in[0], in[st], w);
+    in += 2 * st; w += 8;
+    idct_products(q, in[0], in[st], w);
+#pragma unroll 1
+    for (int k = 4;; k += 2) {
+        in += 2 * st; w += 8;
+        const float2 e = in[0], d = in[st];
+#pragma unroll
+        for (int m = 0; m < 16; ++m) a[m] = add2(a[m], q[m]);
+        idct_products(q, e, d, w);
+        if (k == 14) break;
+    }
+#pragma unroll
+    for (int m = 0; m < 16; ++m) a[m] = add2(a[m], q[m]);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+        o[n] = add2(a[n], a[8 + n]);
+        o[15 - n] = sub2(a[n], a[8 + n]);
     }
 }
 
-// three passes x, y, z over a [z][y][x] cube, ping-ponging a <-> b;
-// result in b. 128 threads, 256 lines x 4 quads per pass.
+// Three passes x, y, z over a block in `buf`, in place; 128 threads, two lines each.
+// In: (z, y, x) at x * 256 + z * 16 + y, stored but not yet synchronised. Out: the
+// thread's values o[z] at y = tid >> 3 and x = 2 * (tid & 7), + 1. The strides keep
+// every load and store of the passes without bank conflicts, but for the x pass's
+// stores (two ways).
+constexpr int kRowX = 256, kRowY = 260, kRowZ = 272;
 template <bool FWD>
-__device__ void transform3(float *a, float *b) {
+__device__ __forceinline__ void transform3(float *buf, float2 o[16]) {
     const int tid = threadIdx.x;
-    for (int t = tid; t < 1024; t += 128) {           // x lines: (z,y)
-        int line = t >> 2, j = t & 3;
-        if (FWD) fdct_quad(a + line * 16, 1, b + line * 16, 1, j);
-        else idct_quad(a + line * 16, 1, b + line * 16, 1, j);
+    float2 *mine = reinterpret_cast<float2 *>(buf) + tid;
+    auto lines = [&](const float2 *in, int st) {
+        if (FWD) dct_lines(in, st, o);
+        else idct_lines(in, st, o);
+    };
+    __syncthreads();
+    lines(mine, kRowX / 2);             // x lines at z = tid >> 3, y = 2 * (tid & 7), + 1
+    __syncthreads();
+    float *to = buf + 2 * (tid & 7) * kRowY + (tid >> 3) * 16;
+#pragma unroll
+    for (int x = 0; x < 16; x += 4) {
+        *reinterpret_cast<float4 *>(to + x) = make_float4(o[x].x, o[x + 1].x, o[x + 2].x, o[x + 3].x);
+        *reinterpret_cast<float4 *>(to + kRowY + x) = make_float4(o[x].y, o[x + 1].y, o[x + 2].y, o[x + 3].y);
     }
     __syncthreads();
-    for (int t = tid; t < 1024; t += 128) {           // y lines: (z,x)
-        int j = t & 3, x = (t >> 2) & 15, z = t >> 6;
-        if (FWD) fdct_quad(b + z * 256 + x, 16, a + z * 256 + x, 16, j);
-        else idct_quad(b + z * 256 + x, 16, a + z * 256 + x, 16, j);
-    }
+    lines(mine, kRowY / 2);             // y lines at z = tid >> 3, x = 2 * (tid & 7), + 1
     __syncthreads();
-    for (int t = tid; t < 1024; t += 128) {           // z lines: (y,x)
-        int j = t & 3, line = t >> 2;
-        if (FWD) fdct_quad(a + line, 256, b + line, 256, j);
-        else idct_quad(a + line, 256, b + line, 256, j);
-    }
+#pragma unroll
+    for (int y = 0; y < 16; ++y) mine[y * (kRowZ / 2)] = o[y];
     __syncthreads();
+    lines(reinterpret_cast<const float2 *>(buf + (tid >> 3) * kRowZ) + (tid & 7), 8);   // z lines
 }
 
 // dead-zone reconstruction (src/mc_codec_float.h:185-190)
@@ -133,8 +179,7 @@ __device__ __forceinline__ float dequant(int lv, int f, const QTab &qt) {
 }
 
 struct EncSmem {
-    float a[kN3];
-    float b[kN3];
+    float a[16 * kRowZ];
     int16_t lv[kN3];
     uint8_t vox[kN3];
     uint32_t mask[4][32];   // entry list and max-error pass: hit masks per warp and step
@@ -145,7 +190,13 @@ struct EncSmem {
 
 }  // namespace
 
-__global__ void __launch_bounds__(128) k_encode(EncParams P) {
+// What bounds it: instruction issue (59 % of the cycles), a quarter of it the
+// transform's packed multiplies and adds, and latency at 5 CTAs (20 warps) per SM. 8
+// chunks at q=6: 0.50 ms; 0.73 ms with one output of one line per step (scalar
+// multiplies and adds, weights indexed by lane, 4-way bank conflicts in the x
+// pass, two 16 KB buffers and 4 CTAs per SM). With the max-error pass (tau=16) 1.04
+// ms against 2.07.
+__global__ void __launch_bounds__(128, 5) k_encode(EncParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     EncSmem &S = *reinterpret_cast<EncSmem *>(smem_raw);
     const int tid = threadIdx.x;
@@ -154,12 +205,14 @@ __global__ void __launch_bounds__(128) k_encode(EncParams P) {
         const EncItem it = P.items[item];
         const QTab &qt = P.qtab[it.qslot];
         const uint8_t *src = reinterpret_cast<const uint8_t *>(it.src);
-        // gather: thread per 16-voxel row
+        // gather: two 16-voxel rows per thread
         uint32_t sum = 0, cnt = 0;
-        for (int r = tid; r < 256; r += 128) {
-            int z = r >> 4, y = r & 15;
+        uint4 rows[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = tid + 128 * h, z = r >> 4, y = r & 15;
             const uint8_t *row = src + z * it.sz + y * it.sy;
-            uint4 w;
+            uint4 &w = rows[h];
             if (((uintptr_t)row & 15) == 0) {
                 w = *reinterpret_cast<const uint4 *>(row);
             } else {
@@ -193,21 +246,30 @@ __global__ void __launch_bounds__(128) k_encode(EncParams P) {
         if (tid == 0 && !cnt) { P.len[item] = 0; P.sym[item] = make_uint2(0, 0); }
         if (!cnt) { __syncthreads(); continue; }       // all air: not coded
         const int dc = (int)((sum + kN3 / 2) / kN3);
-        for (int i = tid; i < kN3; i += 128) S.a[i] = (float)((int)S.vox[i] - dc);
-        __syncthreads();
-        transform3<true>(S.a, S.b);                     // coefficients in S.b
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t ws[4] = {rows[h].x, rows[h].y, rows[h].z, rows[h].w};
+#pragma unroll
+            for (int x = 0; x < 16; ++x)
+                S.a[x * kRowX + tid + 128 * h] = (float)((int)((ws[x >> 2] >> (8 * (x & 3))) & 0xFF) - dc);
+        }
+        float2 o[16];
+        transform3<true>(S.a, o);
         // fused quantiser: t = |c|*rstep + (1-0.8), clamp [0,32767], truncate
         const float bias = 1.0f - 0.80f;
+        const int y0 = tid >> 3, x0 = 2 * (tid & 7);   // the thread's column of coefficients
         uint32_t last = 0;
-        for (int i = tid; i < kN3; i += 128) {
-            float c = S.b[i];
-            int f = (i >> 8) + ((i >> 4) & 15) + (i & 15);
+        auto level = [&](float c, int f) -> uint32_t {
             float t = fadd(fmul(fabsf(c), qt.rstep[f]), bias);
             if (!(t > 0.0f)) t = 0.0f;
             if (!(t < 32767.0f)) t = 32767.0f;
             int v = (int)t;
-            S.lv[i] = (int16_t)(c < 0.0f ? -v : v);
-        }
+            return (uint16_t)(int16_t)(c < 0.0f ? -v : v);
+        };
+#pragma unroll
+        for (int z = 0; z < 16; ++z)
+            reinterpret_cast<uint32_t *>(S.lv)[z * 128 + tid] =
+                level(o[z].x, z + y0 + x0) | level(o[z].y, z + y0 + x0 + 1) << 16;
         __syncthreads();
         // the nonzero levels in scan order as one entry list (position | level
         // << 16) for k_encode_rc: warp w owns positions [1024w, 1024w + 1024) in
@@ -241,12 +303,23 @@ __global__ void __launch_bounds__(128) k_encode(EncParams P) {
         }
         if (it.tau > 0) {
             // local reconstruction for the max-error pass
-            for (int i = tid; i < kN3; i += 128) {
-                int f = (i >> 8) + ((i >> 4) & 15) + (i & 15);
-                S.a[i] = dequant(S.lv[i], f, qt);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = tid + 128 * h;
+                const uint4 *row = reinterpret_cast<const uint4 *>(S.lv + 16 * r);
+                const uint4 u = row[0], v = row[1];
+                const uint32_t ws[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int x = 0; x < 16; ++x)
+                    S.a[x * kRowX + r] =
+                        dequant((int)(int16_t)(ws[x >> 1] >> (16 * (x & 1))), (r >> 4) + (r & 15) + x, qt);
             }
+            transform3<false>(S.a, o);
+            // voxel (z, y, x) to where the thread read (y, z, x) of its own lines
+            float2 *mine = reinterpret_cast<float2 *>(S.a + y0 * kRowZ + x0);
+#pragma unroll
+            for (int z = 0; z < 16; ++z) mine[8 * z] = o[z];
             __syncthreads();
-            transform3<false>(S.a, S.b);                 // reconstruction in S.b
             // corrections in ascending voxel order, written straight to the
             // coder's scratch: warp w owns voxels [1024w, 1024w + 1024) in 32
             // steps of 32; a first pass counts its hits (the step masks kept
@@ -254,7 +327,7 @@ __global__ void __launch_bounds__(128) k_encode(EncParams P) {
             // second pass writes the entries
             const int lane = tid & 31, w = tid >> 5;
             auto hit_at = [&](int i, int &dl) {
-                long long rr = __float2ll_rn(S.b[i]);
+                long long rr = __float2ll_rn(S.a[((i >> 4) & 15) * kRowZ + (i >> 8) * 16 + (i & 15)]);
                 int v = (int)(uint32_t)(unsigned long long)rr + dc;
                 v = v < 0 ? 0 : v > 255 ? 255 : v;
                 const int err = (int)S.vox[i] - v;
@@ -957,7 +1030,11 @@ cudaError_t upload_encode_tables(const float cmf[16][16], const uint16_t scan[kN
     }
     bend[7] = kN3;
     bend[8] = 0xFFFF;
-    const cudaError_t e = cudaMemcpyToSymbolAsync(c_cos, cmf, sizeof(float) * 256, 0, cudaMemcpyHostToDevice, s);
+    float2 fwd[8][16], inv[16][8];
+    for (int k = 0; k < 16; ++k)
+        for (int n = 0; n < 8; ++n) fwd[n][k] = inv[k][n] = make_float2(cmf[k][n], cmf[k][n]);
+    cudaError_t e = cudaMemcpyToSymbolAsync(c_fwd, fwd, sizeof fwd, 0, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(c_inv, inv, sizeof inv, 0, cudaMemcpyHostToDevice, s);
     return e != cudaSuccess ? e : cudaMemcpyToSymbolAsync(c_bend, bend, sizeof bend, 0, cudaMemcpyHostToDevice, s);
 }
 
@@ -997,10 +1074,8 @@ cudaError_t launch_encode(const EncParams &p, cudaStream_t s) {
     });
     if (a < 0) return (cudaError_t)(-a);
     const int sms = dev_sms();
-    // one wave of CTAs: as many per SM as fit (45.6 KB of shared memory plus
-    // the per-CTA reserve, in allocation units, leaves room for 4). CTAs walk
-    // the blocks with a fixed stride, so CTAs beyond one wave would start
-    // their whole share late.
+    // one wave of CTAs: as many per SM as fit. CTAs walk the blocks with a fixed
+    // stride, so CTAs beyond one wave would start their whole share late.
     static std::atomic<int> occ_by_dev[kMaxDevs];
     const int occ = dev_once(occ_by_dev, [smem] {
         int o = 0;

@@ -113,7 +113,7 @@ struct Lane {
     DevBuf solo;                                // single-block decode scratch (SoloScratch)
     HostBuf h_items, h_base, h_stage, h_misc;
     HostBuf h_one;                              // single-block output, written by the kernel over the bus
-    HostBuf h_bounce[3];                        // device-to-host pieces bound for pageable memory
+    HostBuf h_bounce[3];                        // pieces between the device and pageable memory
     cudaEvent_t bounce_ev[3] = {};
     LaunchCfg cfg;
     BlobSlot pipe[kBlobSlots];
