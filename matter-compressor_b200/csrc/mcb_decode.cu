@@ -1349,12 +1349,16 @@ __global__ void __launch_bounds__(64, 9) k_reconstruct(RecParams P) {
     for (int i = tid; i < kBoxB / 4; i += 64) reinterpret_cast<float4 *>(S.box)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     const int nb = gridDim.x;
+    // blocks dealt to the CTAs in turn; in a large batch two adjacent ones at a
+    // time, so that the two halves of a 32-byte sector of the output are written
+    // soon after one another (see launch_reconstruct)
+    auto after = [&P, nb](int j) { return !P.pairs ? j + nb : (j & 1 ? j + 2 * nb - 1 : j + 1); };
     const int mh = lane & 3, m = mh * 2;
     float *const A = S.a[warp];
     uint8_t *const stage = reinterpret_cast<uint8_t *>(S.a);
     // the next block's header, entry offset and payload length, loaded while
     // this one is transformed; then its first 256 entries, while pass 3 runs
-    int i = blockIdx.x;
+    int i = P.pairs ? 2 * blockIdx.x : blockIdx.x;
     EntHdr hn = {};
     uint64_t basen = 0;
     uint32_t lenn = 0, slotn = 0, en[4] = {0, 0, 0, 0};
@@ -1376,13 +1380,14 @@ __global__ void __launch_bounds__(64, 9) k_reconstruct(RecParams P) {
         next_head(i);
         next_entries();
     }
-    for (; i < P.n; i += nb) {
+    for (int nx; i < P.n; i = nx) {
+        nx = after(i);
         const int item = P.idx ? (int)__ldg(P.idx + i) : i;
         const DecItem it = P.items[item];
         const EntHdr h = hn;
         const uint64_t base = basen;
         const uint32_t len = lenn, cap = entry_cap(lenn), nslot = slotn;
-        if (i + nb < P.n) next_head(i + nb);
+        if (nx < P.n) next_head(nx);
         // the header comes from k_entropy; the guards keep every index below
         // inside shared memory whatever its contents
         const bool sane = h.nnz <= kN3 && h.ncorr <= kN3;
@@ -1397,13 +1402,13 @@ __global__ void __launch_bounds__(64, 9) k_reconstruct(RecParams P) {
                 uint8_t *dst = reinterpret_cast<uint8_t *>(it.dst) + (tid & 15) * it.sy + (tid >> 4) * it.sz;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) store_row16(dst + 4 * j * it.sz, make_uint4(w, w, w, w));
-                if (i + nb < P.n) next_entries();
+                if (nx < P.n) next_entries();
                 continue;
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 reinterpret_cast<uint4 *>(stage + warp * kStageHalf)[j * 32 + lane] = make_uint4(w, w, w, w);
-            if (i + nb < P.n) next_entries();
+            if (nx < P.n) next_entries();
         } else {
             // one pass over the entries, as in reconstruct_block
             const QTab &qt = P.qtab[nslot];
@@ -1496,7 +1501,7 @@ __global__ void __launch_bounds__(64, 9) k_reconstruct(RecParams P) {
                 }
                 __syncwarp();
             }
-            if (i + nb < P.n) next_entries();
+            if (nx < P.n) next_entries();
             __syncthreads();   // every plane has its pass-2 output
             // pass 3: lane l of warp w takes the group (y, xg) = (8 w + (l >> 2), l & 3)
             const int y = 8 * warp + (lane >> 2);
@@ -1933,7 +1938,15 @@ cudaError_t launch_reconstruct(const RecParams &p, const LaunchCfg &cfg, cudaStr
         return e == cudaSuccess ? 1 : -(int)e;
     });
     if (a < 0) return (cudaError_t)(-a);
-    k_reconstruct<<<blocks, 64, sizeof(RecSmem), s>>>(p);
+    // From 64 blocks per CTA up, where the output is several times the L2 and a
+    // CTA's turn comes round late: half-written sectors then leave the L2 and are
+    // read back and written twice (16 chunks, 268 MB: 213 MB read and 380 written).
+    // 64 chunks at q=6 1.55 ms against 1.61, q=1 3.52 against 3.63. Below that the
+    // batch is cut less evenly than by single blocks: 8 chunks at q=3 350 us
+    // against 336, 3 chunks at q=12 73 against 72.
+    RecParams P = p;
+    P.pairs = p.n >= 64 * blocks;
+    k_reconstruct<<<blocks, 64, sizeof(RecSmem), s>>>(P);
     return cudaGetLastError();
 }
 

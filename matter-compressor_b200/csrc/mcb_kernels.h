@@ -61,6 +61,7 @@ struct RecParams {
     const uint32_t *pool;
     const QTab *qtab;
     const uint16_t *scan;      // scan position -> raster idx | band<<12
+    bool pairs = false;        // set by the launcher: a CTA takes two adjacent blocks at a time
 };
 
 // Both stages in one persistent kernel: entropy lanes mark finished blocks

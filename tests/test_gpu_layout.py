@@ -1,7 +1,9 @@
 """The batch layout made on the device (arena ranges and processing order), at
 item counts around its CTAs' 1024 items and with every length class in use:
-absent blocks, the shortest payloads and ones past 4092 bytes. Whole numbers:
-equality with the oracle's block decoder."""
+absent blocks, the shortest payloads and ones past 4092 bytes; and the
+reconstruction's dealing of blocks to CTAs, one or two at a time, around the
+count where it changes. Whole numbers: equality with the oracle's block
+decoder."""
 import numpy as np
 import pytest
 
@@ -49,3 +51,20 @@ def test_nothing_coded(chunk):
                               out.data_ptr(), 4096) == 0
     torch.cuda.synchronize()
     assert not out.any()
+
+
+@pytest.mark.parametrize("over", [-1, 0, 1, 2, 2 * 9 * 148 + 1])
+def test_blocks_per_cta(chunk, over):
+    """Around 64 blocks for each of the reconstruction's CTAs (9 per SM)."""
+    import torch
+    a, pick, want = chunk
+    n = 64 * 9 * torch.cuda.get_device_properties(0).multi_processor_count + over
+    short = np.flatnonzero(pick < 20)     # payloads of a few dozen bytes: one batch holds them all
+    at = short[np.random.default_rng(5).integers(0, len(short), n)]
+    boxes = [(16 * int(b >> 8), 16 * int(b >> 4 & 15), 16 * int(b & 15)) for b in at]
+    out = torch.full((n + 1, 4096), 0xA7, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    assert a.read_regions_dev(0, boxes, 16, 16, 16, out.data_ptr(), 4096) == 0
+    torch.cuda.synchronize()
+    ref = torch.from_numpy(want.reshape(-1, 4096)).cuda()[torch.from_numpy(pick[at]).cuda()]
+    assert torch.equal(out[:n], ref) and bool((out[n] == 0xA7).all())
