@@ -198,7 +198,7 @@ __device__ __forceinline__ void db_filter16h(const uint4 P1, uint4 &P0, uint4 &Q
 // chunks (268 MB): 85 us (a copy takes 86), 141 us as three passes (the x pass
 // alone moves every sector both ways); with the faces in integers 122 us, the ALU
 // pipe 82 % busy.
-constexpr uint32_t kTileMaxVecs = 64;   // row length of at most 1024: 512 threads
+constexpr uint32_t kTileMaxVecs = 56;   // row vectors: 448 threads
 
 __global__ void __launch_bounds__(kTileMaxVecs * 8) k_deblock_tile(DbParams P, uint32_t ty) {
     extern __shared__ __align__(16) uint8_t s_db[];
@@ -305,8 +305,19 @@ cudaError_t launch_deblock(uint8_t *d_vol, int count, size_t vstride, int nz, in
     // voxel.)
     const uint32_t ty = (uint32_t)(((uint64_t)ny + 11) / 8), tz = (uint32_t)(((uint64_t)nz + 11) / 8);
     const uint64_t tiles = (uint64_t)ty * tz;
-    if (vec && beta <= kHalfBeta && (uint32_t)nx <= 16 * kTileMaxVecs && !(ny > 16 && ny % 16 == 1) && tiles < (1ull << 31)) {
-        const uint32_t nseg = (uint32_t)nx / 16;
+    // And where the tiles do not cost more than the passes they save. Without y and
+    // z faces the passes leave most rows alone (4096 volumes of 512 x 1 x 16: 16 us,
+    // 148 as tiles). Otherwise the tiles' work, warps filled up and rows beyond the
+    // edges counted, may be 1.9 times the volume's at row lengths of 64 to 576 and 1.5
+    // times elsewhere (400 MB of volumes, tiles / passes: 24 x 24 x 128 at 1.78 times
+    // 0.94, 48 x 48 x 96 at 1.81 1.00, 24 x 24 x 96 at 2.37 1.17, 256 x 256 x 32 at 2.12
+    // 1.20, 24 x 24 x 640 at 1.78 1.12, 40 x 40 x 640 at 1.44 0.95, 256 x 256 x 48 at
+    // 1.41 0.91). CTAs for longer rows fit an SM one fewer at a time (256 x 256 x 896:
+    // 0.78, 944: 1.06, 1024: 1.02; 40 x 40: 0.88, 1.26, 1.19).
+    const uint32_t nseg = (uint32_t)nx / 16;
+    const uint64_t work = tiles * 64 * (uint64_t)((nseg * 8 + 31) / 32 * 64);
+    const bool pays = ny > 16 && nz > 16 && 10 * work <= (nx >= 64 && nx <= 576 ? 19u : 15u) * P.total;
+    if (vec && beta <= kHalfBeta && nseg <= kTileMaxVecs && !(ny % 16 == 1) && pays && tiles < (1ull << 31)) {
         const size_t smem = (size_t)nseg * (4 * 8 * sizeof(uint4) + 8 * 8 * sizeof(uint32_t));   // 768 B a vector
         k_deblock_tile<<<dim3((unsigned)tiles, (unsigned)count), nseg * 8, smem, s>>>(P, ty);
         return cudaGetLastError();
