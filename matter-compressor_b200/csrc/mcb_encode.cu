@@ -418,10 +418,6 @@ __device__ __forceinline__ uint32_t code_norm(EncLane &e) {
     e.n += s >> 3;
     return s;
 }
-__device__ __forceinline__ void put_byte(EncLane &e, uint32_t b) {
-    if (e.len < (uint32_t)kEncCap) e.out[e.len] = (uint8_t)b;
-    ++e.len;
-}
 // A carry past the held bytes: one more in the bytes already written.
 __device__ __noinline__ void code_carry(uint8_t *out, uint32_t len) {
     uint32_t i = min(len, (uint32_t)kEncCap);
@@ -446,19 +442,51 @@ __device__ __forceinline__ void code_settle(EncLane &e) {   // after a single op
     while (e.range < kEncTop) code_norm(e);
     while (e.n >= 4) code_flush(e);
 }
-__device__ __forceinline__ void code_bin(EncLane &e, uint32_t *c, uint32_t bit) {
-    const uint32_t p0 = *c, r0 = (e.range >> 12) * p0;
-    if (!bit) { e.range = r0; *c = p0 + ((4096u - p0) >> 4); }
-    else { code_add(e, r0); e.range -= r0; *c = p0 - (p0 >> 4); }
+
+// The coder of a thread that is alone on its warp: the held bytes and low in one
+// 64-bit word, 1 to 3 bytes held, a byte at a time.
+struct EncOne {
+    uint8_t *out;
+    uint32_t len, n, range;
+    uint64_t code;   // n held bytes, low
+};
+__device__ __forceinline__ void code_add(EncOne &e, uint32_t v) { e.code += v; }
+__device__ __forceinline__ void code_settle(EncOne &e) {
+    while (e.range < kEncTop) {
+        if (e.n == 3) {   // the two oldest go out
+            const uint32_t v = (uint32_t)(e.code >> 40);
+            e.code &= (1ull << 40) - 1u;
+            e.n = 1;
+            if (v >> 16) code_carry(e.out, e.len);
+            if (e.len + 2 <= (uint32_t)kEncCap)   // even offsets, even base
+                *reinterpret_cast<uint16_t *>(e.out + e.len) = (uint16_t)((v >> 8 & 0xFFu) | (v & 0xFFu) << 8);
+            e.len += 2;
+        }
+        e.code <<= 8;
+        e.range <<= 8;
+        ++e.n;
+    }
+}
+
+// Single bins of either coder.
+__device__ __forceinline__ uint32_t after0(uint32_t p) { return p + ((4096u - p) >> 4); }
+__device__ __forceinline__ uint32_t after1(uint32_t p) { return p - (p >> 4); }
+template <class Coder>
+__device__ __forceinline__ void code_bin(Coder &e, uint32_t &p0, uint32_t bit) {
+    const uint32_t r0 = (e.range >> 12) * p0;
+    if (!bit) { e.range = r0; p0 = after0(p0); }
+    else { code_add(e, r0); e.range -= r0; p0 = after1(p0); }
     code_settle(e);
 }
-__device__ __forceinline__ void code_bypass(EncLane &e, uint32_t bit) {
+template <class Coder>
+__device__ __forceinline__ void code_bypass(Coder &e, uint32_t bit) {
     e.range >>= 1;
     if (bit) code_add(e, e.range);
     code_settle(e);
 }
 // k bits MSB-first, 16 at a time from the top (src/mc_codec.c:209-215)
-__device__ __forceinline__ void code_bits(EncLane &e, uint32_t v, int k) {
+template <class Coder>
+__device__ __forceinline__ void code_bits(Coder &e, uint32_t v, int k) {
     while (k > 0) {
         const int take = k > 16 ? 16 : k;
         e.range >>= take;
@@ -468,12 +496,56 @@ __device__ __forceinline__ void code_bits(EncLane &e, uint32_t v, int k) {
     }
 }
 // order-0 Exp-Golomb (src/mc_codec.c:229-233)
-__device__ __forceinline__ void code_eg(EncLane &e, uint32_t v) {
+template <class Coder>
+__device__ __forceinline__ void code_eg(Coder &e, uint32_t v) {
     const uint32_t t = v + 1u;
     const int nb = bitlen32(t) - 1;
     for (int i = 0; i < nb; ++i) code_bypass(e, 1);
     code_bypass(e, 0);
     if (nb > 0) code_bits(e, t & ((1u << nb) - 1u), nb);
+}
+// Header bins and EOB: its bit length prefix, then the bits below the MSB
+// (src/mc_codec.c:314-320). No context occurs twice; p0(j) is context j's.
+template <class Coder, class P0>
+__device__ __forceinline__ void code_header(Coder &e, P0 p0, uint32_t dc, uint32_t eob, uint32_t ncorr) {
+    auto bin = [&](int j, uint32_t bit) {
+        uint32_t p = p0(j);
+        code_bin(e, p, bit);
+    };
+    bin(kCtxFlag + 0, 0);                 // reserved
+    bin(kCtxFlag + 1, ncorr > 0);
+    for (int b = 0; b < 8; ++b) bin(kCtxDc + b, (dc >> (7 - b)) & 1);
+    const int k = bitlen32(eob);
+    for (int i = 0; i < k; ++i) bin(kCtxEob + i, 1);
+    if (k < 13) bin(kCtxEob + k, 0);
+    if (k > 1) code_bits(e, eob & ((1u << (k - 1)) - 1u), k - 1);
+}
+// What follows the scan (src/mc_codec.c:721-729).
+template <class Coder>
+__device__ __forceinline__ void code_corrections(Coder &e, const uint32_t *cor, uint32_t ncorr) {
+    if (!ncorr) return;
+    code_eg(e, ncorr - 1);
+    uint32_t prev = 0;
+    for (uint32_t c = 0; c < ncorr; ++c) {
+        const uint32_t w = cor[c];
+        const uint32_t pos = w & 0xFFFF;
+        code_eg(e, pos - prev);
+        prev = pos;
+        const int d = (int16_t)(w >> 16);
+        code_bypass(e, d < 0);
+        code_eg(e, (uint32_t)(d < 0 ? -d : d) - 1u);
+    }
+}
+// The n held bytes, then the four of low; the payload's length.
+__device__ __forceinline__ void code_end(const EncParams &P, int item, uint8_t *out, uint32_t len, uint64_t held,
+                                         uint32_t n, uint32_t low) {
+    if ((held >> (8 * n)) & 1) code_carry(out, len);
+    for (int i = (int)n + 3; i >= 0; --i, ++len) {
+        const uint32_t b = i >= 4 ? (uint32_t)(held >> (8 * (i - 4))) : low >> (8 * i);
+        if (len < (uint32_t)kEncCap) out[len] = (uint8_t)b;
+    }
+    if (len > (uint32_t)kEncCap) atomicAdd(P.status, 1u);
+    P.len[item] = min(len, (uint32_t)kEncCap);
 }
 
 __device__ __forceinline__ void enc_density(EncLane &e) {
@@ -502,7 +574,7 @@ __device__ __forceinline__ void enc_position(EncLane &e, uint32_t *ctx, const ui
     while (e.p >= e.bend) { e.band++; e.sigb += 4; e.bend = s_bend[e.band]; }
     if (e.p + 1 >= e.eob) {
         for (uint32_t k = 0; k < 12u; ++k) {
-            code_bin(e, ctx + (kCtxMag + k) * 32, k < e.kend);
+            code_bin(e, ctx[(kCtxMag + k) * 32], k < e.kend);
             if (k >= e.kend) break;
         }
         if (e.m > 12u) code_eg(e, e.m - 12u);
@@ -614,14 +686,7 @@ __global__ void __launch_bounds__(kRcWarps * 32) k_encode_rc(EncParams P, int la
             e.out = reinterpret_cast<uint8_t *>(it.out);
             for (int j = 0; j < kNumCtx; ++j) ctx[j * 32] = qt.ctx[j];
             ctx[kEncScr * 32] = 1;
-            code_bin(e, ctx + (kCtxFlag + 0) * 32, 0);                 // reserved
-            code_bin(e, ctx + (kCtxFlag + 1) * 32, ncorr > 0);
-            for (int b = 0; b < 8; ++b) code_bin(e, ctx + (kCtxDc + b) * 32, (dc >> (7 - b)) & 1);
-            // EOB: bit length prefix then the bits below the MSB (src/mc_codec.c:314-320)
-            const int k = bitlen32(eob);
-            for (int i = 0; i < k; ++i) code_bin(e, ctx + (kCtxEob + i) * 32, 1);
-            if (k < 13) code_bin(e, ctx + (kCtxEob + k) * 32, 0);
-            if (k > 1) code_bits(e, eob & ((1u << (k - 1)) - 1u), k - 1);
+            code_header(e, [ctx](int j) { return ctx[j * 32]; }, dc, eob, ncorr);
             if (eob) {
                 e.ent = P.entries + (size_t)item * kN3;
                 e.eob = eob;
@@ -645,30 +710,130 @@ __global__ void __launch_bounds__(kRcWarps * 32) k_encode_rc(EncParams P, int la
             }
         }
         if (coded) {
-            if (ncorr) {                                     // src/mc_codec.c:721-729
-                const uint32_t *cor = P.corr + (size_t)item * kN3;
-                code_eg(e, ncorr - 1);
-                uint32_t prev = 0;
-                for (uint32_t c = 0; c < ncorr; ++c) {
-                    const uint32_t w = cor[c];
-                    const uint32_t pos = w & 0xFFFF;
-                    code_eg(e, pos - prev);
-                    prev = pos;
-                    const int d = (int16_t)(w >> 16);
-                    code_bypass(e, d < 0);
-                    code_eg(e, (uint32_t)(d < 0 ? -d : d) - 1u);
-                }
-            }
-            // the held bytes, then the four of low
-            const uint64_t acc = (uint64_t)e.ah << 32 | e.al;
-            if ((acc >> (8 * e.n)) & 1) code_carry(e.out, e.len);
-            for (int i = (int)e.n - 1; i >= 0; --i) put_byte(e, (uint32_t)(acc >> (8 * i)) & 0xFFu);
-            for (int i = 3; i >= 0; --i) put_byte(e, (e.low >> (8 * i)) & 0xFFu);
-            if (e.len > (uint32_t)kEncCap) atomicAdd(P.status, 1u);
-            P.len[item] = min(e.len, (uint32_t)kEncCap);
+            code_corrections(e, P.corr + (size_t)item * kN3, ncorr);
+            code_end(P, item, e.out, e.len, (uint64_t)e.ah << 32 | e.al, e.n, e.low);
         }
         __syncwarp();
     }
+}
+
+// The coder of a few blocks, each by one thread alone on its warp: the mirror of
+// the decoder's solo_entropy (mcb_decode.cu). The contexts of the scan are held in
+// registers, the four of the current band and the twelve rungs, and every
+// position jumps to where the next is coded; a run of zeros in a sparse density
+// class goes four at a time, one compare of the last split deciding that none
+// renormalises. What bounds it: the chain of dependent instructions through the
+// range. A block of noise at q=0.5 takes 2.57 ms, 10.1 as the one live lane of
+// k_encode_rc, which pays every lane's step for it (3.54 bin by bin from a list of
+// levels); textured material at q=24 130 us, 204 and 500.
+namespace {
+__device__ __forceinline__ bool code_rung(EncOne &e, uint32_t &g, bool up) {
+    code_bin(e, g, up);
+    return up;
+}
+__device__ __forceinline__ void code_scan(EncOne &e, const QTab &qt, const uint32_t *ent, uint32_t eob) {
+    uint32_t g0 = qt.ctx[kCtxMag + 0], g1 = qt.ctx[kCtxMag + 1], g2 = qt.ctx[kCtxMag + 2], g3 = qt.ctx[kCtxMag + 3];
+    uint32_t g4 = qt.ctx[kCtxMag + 4], g5 = qt.ctx[kCtxMag + 5], g6 = qt.ctx[kCtxMag + 6], g7 = qt.ctx[kCtxMag + 7];
+    uint32_t g8 = qt.ctx[kCtxMag + 8], g9 = qt.ctx[kCtxMag + 9], g10 = qt.ctx[kCtxMag + 10], g11 = qt.ctx[kCtxMag + 11];
+    uint32_t s0 = 0, s1 = 0, s2 = 0, s3 = 0;   // the band's contexts
+    uint32_t p = 0, e1 = 0, e2 = 0, e3 = 0, band = 0, bend = 0, stop = 0;
+    uint32_t w = ent[0], ahead = ent[1], idx = 2, pos = w & 0xFFFFu;
+    auto to_band = [&](uint32_t b) {
+        band = b;
+        bend = c_bend[b];
+        const uint16_t *c = qt.ctx + kCtxSig + 4 * b;
+        s0 = c[0]; s1 = c[1]; s2 = c[2]; s3 = c[3];
+    };
+    to_band(0);
+position:   // a band change, or the last position, significant by definition
+    while (p >= bend) to_band(band + 1);
+    stop = min(bend, eob - 1);
+    if (p + 1 == eob) {
+        ++p;
+        goto coef;
+    }
+next:       // a significance bin at p < stop
+    if (p < e3) {   // density class 3: bins one at a time
+        const bool sig = p == pos;
+        code_bin(e, s3, sig);
+        ++p;
+        if (sig) goto one;
+        if (p >= stop) goto position;
+        goto next;
+    } else {
+        const bool a2 = p < e2, a1 = p < e1;
+        const uint32_t lim = min(stop, a2 ? e2 : (a1 ? e1 : 0xFFFFFFFFu)), end = min(lim, pos);
+        uint32_t pc = a2 ? s2 : (a1 ? s1 : s0);
+        while (p < end) {
+            if (p + 4u <= end) {
+                const uint32_t r1 = (e.range >> 12) * pc, q1 = after0(pc);
+                const uint32_t r2 = (r1 >> 12) * q1, q2 = after0(q1);
+                const uint32_t r3 = (r2 >> 12) * q2, q3 = after0(q2);
+                const uint32_t r4 = (r3 >> 12) * q3;
+                if (r4 >= kEncTop) {
+                    e.range = r4;
+                    pc = after0(q3);
+                    p += 4;
+                    continue;
+                }
+            }
+            code_bin(e, pc, 0);
+            ++p;
+        }
+        const bool sig = p < lim;   // p is the next significant position
+        if (sig) {
+            code_bin(e, pc, 1);
+            ++p;
+        }
+        s0 = a1 ? s0 : pc;
+        s1 = a1 & !a2 ? pc : s1;
+        s2 = a2 ? pc : s2;
+        if (sig) goto one;
+        if (p >= stop) goto position;
+        goto next;
+    }
+one:
+    e3 = e2;
+    e2 = e1;
+    e1 = p + 16u;
+coef:       // the coefficient at p - 1 (src/mc_codec.c:268-275)
+    {
+        const int lv = (int)w >> 16;
+        const uint32_t m = (uint32_t)(lv < 0 ? -lv : lv);
+        w = ahead;
+        pos = w & 0xFFFFu;
+        ahead = ent[min(idx, (uint32_t)kN3 - 1u)];
+        ++idx;
+        if (code_rung(e, g0, m > 1) && code_rung(e, g1, m > 2) && code_rung(e, g2, m > 3) && code_rung(e, g3, m > 4) &&
+            code_rung(e, g4, m > 5) && code_rung(e, g5, m > 6) && code_rung(e, g6, m > 7) && code_rung(e, g7, m > 8) &&
+            code_rung(e, g8, m > 9) && code_rung(e, g9, m > 10) && code_rung(e, g10, m > 11) &&
+            code_rung(e, g11, m > 12))
+            code_eg(e, m - 12u);
+        code_bypass(e, lv < 0);
+    }
+    if (p >= eob) return;
+    if (p < stop) goto next;
+    goto position;
+}
+}  // namespace
+__global__ void __launch_bounds__(32) k_encode_rc_one(EncParams P) {
+    const int item = blockIdx.x;
+    if (threadIdx.x) return;
+    const uint2 sy = P.sym[item];
+    if (!(sy.x & 0x80000000u)) return;   // all air: not coded
+    const uint32_t dc = sy.x & 0xFF, eob = (sy.x >> 8) & 0x1FFF, ncorr = sy.y;
+    const EncItem it = P.items[item];
+    const QTab &qt = P.qtab[it.qslot];
+    EncOne e;
+    e.out = reinterpret_cast<uint8_t *>(it.out);
+    e.len = 0;
+    e.n = 1;   // the coder's leading byte
+    e.range = 0xFFFFFFFFu;
+    e.code = 0;
+    code_header(e, [&qt](int j) { return (uint32_t)qt.ctx[j]; }, dc, eob, ncorr);
+    if (eob) code_scan(e, qt, P.entries + (size_t)item * kN3, eob);
+    code_corrections(e, P.corr + (size_t)item * kN3, ncorr);
+    code_end(P, item, e.out, e.len, e.code >> 32, e.n, (uint32_t)e.code);
 }
 
 // ------------------------------------------------------------ blob assembly
@@ -709,12 +874,10 @@ __global__ void __launch_bounds__(256) k_frac_count(EncParams P) {
 // computed one from the other, when the last range shows that none of them
 // renormalises. One chunk or many: 0.95 ms as the tail of the sizing pass with
 // contexts in local memory, 0.75 ms here and hidden.
-__device__ __forceinline__ uint32_t up0(uint32_t p) { return p + ((4096u - p) >> 4); }
-__device__ __forceinline__ uint32_t up1(uint32_t p) { return p - (p >> 4); }
 __device__ __forceinline__ void frac_bit(Enc &e, uint32_t &p0, uint32_t bit) {
     const uint32_t r0 = (e.range >> 12) * p0;
-    if (!bit) { e.range = r0; p0 = up0(p0); }
-    else { e.low += r0; e.range -= r0; p0 = up1(p0); }
+    if (!bit) { e.range = r0; p0 = after0(p0); }
+    else { e.low += r0; e.range -= r0; p0 = after1(p0); }
     enc_norm(e);
 }
 __device__ __forceinline__ void frac_nibble(Enc &e, uint32_t (&p)[4], uint32_t v) {
@@ -750,7 +913,7 @@ __global__ void __launch_bounds__(32) k_fracmap(BlobParams P) {
                     const uint32_t r3 = (r2 >> 12) * lo[1], r4 = (r3 >> 12) * lo[0];
                     if (v == 0 && r4 >= (1u << 24)) {
                         e.range = r4;
-                        lo[3] = up0(lo[3]); lo[2] = up0(lo[2]); lo[1] = up0(lo[1]); lo[0] = up0(lo[0]);
+                        lo[3] = after0(lo[3]); lo[2] = after0(lo[2]); lo[1] = after0(lo[1]); lo[0] = after0(lo[0]);
                     } else {
                         frac_nibble(e, lo, v);
                     }
@@ -762,7 +925,7 @@ __global__ void __launch_bounds__(32) k_fracmap(BlobParams P) {
                     if (v == 15 && r4 >= (1u << 24)) {
                         e.low += (uint64_t)s1 + s2 + s3 + s4;
                         e.range = r4;
-                        hi[3] = up1(hi[3]); hi[2] = up1(hi[2]); hi[1] = up1(hi[1]); hi[0] = up1(hi[0]);
+                        hi[3] = after1(hi[3]); hi[2] = after1(hi[2]); hi[1] = after1(hi[1]); hi[0] = after1(hi[0]);
                     } else {
                         frac_nibble(e, hi, v);
                     }
@@ -1089,10 +1252,14 @@ cudaError_t launch_encode(const EncParams &p, cudaStream_t s) {
 
 cudaError_t launch_encode_rc(const EncParams &p, cudaStream_t s) {
     if (p.n <= 0) return cudaSuccess;
-    // at least one warp for each of the SMs' four schedulers while a warp
+    // otherwise at least one warp for each of the SMs' four schedulers while a warp
     // still has four blocks or more (8 chunks at q=6: 0.97 ms with 32 lanes, 1.36
     // with 16; 2 chunks at q=1 tau=4: 5.06, 4.41, and 4.39 with 8)
     const int sms = dev_sms();
+    if (p.n <= sms) {   // as many blocks as SMs or fewer, the single-block call: a thread and a CTA each
+        k_encode_rc_one<<<p.n, 32, 0, s>>>(p);
+        return cudaGetLastError();
+    }
     int lanes = 32;
     while (lanes > 4 && p.n < lanes * sms * 4) lanes >>= 1;
     const int blocks = ((p.n + lanes - 1) / lanes + kRcWarps - 1) / kRcWarps;
