@@ -17,6 +17,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "mcb_devinfo.h"
 #include "mcb_f32x2.cuh"
 #include "mcb_format.h"
@@ -184,8 +186,9 @@ struct EncSmem {
     uint8_t vox[kN3];
     uint32_t mask[4][32];   // entry list and max-error pass: hit masks per warp and step
     uint32_t red[8];
-    uint32_t ncorr;
+    uint32_t ncorr, nent;
     uint32_t eob;
+    uint32_t used;   // words of the CTA's share of the pool that hold symbols
 };
 
 }  // namespace
@@ -200,6 +203,19 @@ __global__ void __launch_bounds__(128, 5) k_encode(EncParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     EncSmem &S = *reinterpret_cast<EncSmem *>(smem_raw);
     const int tid = threadIdx.x;
+    // the CTA's share of the symbol pool, filled block after block. A block that
+    // it has no room for is left out and counted in status[1]: the caller runs the
+    // launch again with a larger pool.
+    const uint32_t share = P.pool_words / gridDim.x, pool0 = blockIdx.x * share;
+    if (tid == 0) S.used = 0;
+    auto no_room = [&](int item) {
+        if (tid == 0) {
+            atomicAdd(P.status + 1, 1u);
+            P.len[item] = 0;
+            P.sym[item] = make_uint4(0, 0, 0, 0);
+        }
+        __syncthreads();
+    };
 
     for (int item = blockIdx.x; item < P.n; item += gridDim.x) {
         const EncItem it = P.items[item];
@@ -243,7 +259,7 @@ __global__ void __launch_bounds__(128, 5) k_encode(EncParams P) {
         __syncthreads();
         sum = S.red[0] + S.red[1] + S.red[2] + S.red[3];
         cnt = S.red[4] + S.red[5] + S.red[6] + S.red[7];
-        if (tid == 0 && !cnt) { P.len[item] = 0; P.sym[item] = make_uint2(0, 0); }
+        if (tid == 0 && !cnt) { P.len[item] = 0; P.sym[item] = make_uint4(0, 0, 0, 0); }
         if (!cnt) { __syncthreads(); continue; }       // all air: not coded
         const int dc = (int)((sum + kN3 / 2) / kN3);
 #pragma unroll
@@ -292,7 +308,13 @@ __global__ void __launch_bounds__(128, 5) k_encode(EncParams P) {
             __syncthreads();
             uint32_t at = 0;
             for (int ww = 0; ww < w; ++ww) at += S.red[ww];
-            uint32_t *ent = P.entries + (size_t)item * kN3;
+            const uint32_t nent = S.red[0] + S.red[1] + S.red[2] + S.red[3];
+            if (S.used + nent > share) {
+                no_room(item);
+                continue;
+            }
+            if (tid == 0) S.nent = nent;
+            uint32_t *ent = P.pool + pool0 + S.used;
             for (int k = 0; k < 32; ++k) {
                 const uint32_t m = S.mask[w][k], p = 1024u * w + 32u * k + lane;
                 if ((m >> lane) & 1)
@@ -346,7 +368,12 @@ __global__ void __launch_bounds__(128, 5) k_encode(EncParams P) {
             __syncthreads();
             uint32_t at = 0;
             for (int ww = 0; ww < w; ++ww) at += S.red[ww];
-            uint32_t *cor = P.corr + (size_t)item * kN3;
+            const uint32_t ncorr = S.red[0] + S.red[1] + S.red[2] + S.red[3], cor0 = S.used + S.nent;
+            if (cor0 + ncorr > share) {
+                no_room(item);
+                continue;
+            }
+            uint32_t *cor = P.pool + pool0 + cor0;
             for (int k = 0; k < 32; ++k) {
                 const uint32_t m = S.mask[w][k];
                 if ((m >> lane) & 1) {
@@ -357,11 +384,14 @@ __global__ void __launch_bounds__(128, 5) k_encode(EncParams P) {
                 }
                 at += __popc(m);
             }
-            if (tid == 0) S.ncorr = S.red[0] + S.red[1] + S.red[2] + S.red[3];
+            if (tid == 0) S.ncorr = ncorr;
         }
-        __syncthreads();   // ncorr complete
-        // (dc, eob) with the coded flag, ncorr
-        if (tid == 0) P.sym[item] = make_uint2(0x80000000u | (S.eob << 8) | (uint32_t)dc, S.ncorr);
+        __syncthreads();   // nent and ncorr complete, used read
+        if (tid == 0) {
+            const uint32_t at = pool0 + S.used;
+            P.sym[item] = make_uint4(0x80000000u | (S.eob << 8) | (uint32_t)dc, S.ncorr, at, at + S.nent);
+            S.used += S.nent + S.ncorr;
+        }
         __syncthreads();
     }
 }
@@ -564,8 +594,7 @@ __device__ __forceinline__ void set_entry(EncLane &e, uint32_t w) {
 }
 __device__ __forceinline__ void next_entry(EncLane &e) {
     set_entry(e, e.ahead);
-    e.ahead = e.ent[min(e.idx, (uint32_t)kN3 - 1u)];
-    ++e.idx;
+    e.ahead = e.ent[e.idx++];   // up to two entries past the block's last (EncParams::pool)
 }
 // p >= stop: a band change, or the last position, significant by definition:
 // its coefficient without a significance bin (src/mc_codec.c:337-349); the
@@ -669,7 +698,7 @@ __global__ void __launch_bounds__(kRcWarps * 32) k_encode_rc(EncParams P, int la
     const int ngroups = (P.n + lanes - 1) / lanes;
     for (int g = blockIdx.x * kRcWarps + warp; g < ngroups; g += gridDim.x * kRcWarps) {
         const int item = g * lanes + lane;
-        uint2 sy = make_uint2(0, 0);
+        uint4 sy = make_uint4(0, 0, 0, 0);
         if (lane < lanes && item < P.n) sy = P.sym[item];
         const bool coded = (sy.x & 0x80000000u) != 0;   // an all-air block is not coded
         const uint32_t dc = sy.x & 0xFF, eob = (sy.x >> 8) & 0x1FFF, ncorr = sy.y;
@@ -688,7 +717,7 @@ __global__ void __launch_bounds__(kRcWarps * 32) k_encode_rc(EncParams P, int la
             ctx[kEncScr * 32] = 1;
             code_header(e, [ctx](int j) { return ctx[j * 32]; }, dc, eob, ncorr);
             if (eob) {
-                e.ent = P.entries + (size_t)item * kN3;
+                e.ent = P.pool + sy.z;
                 e.eob = eob;
                 e.sigb = kCtxSig;
                 e.bend = s_bend[0];
@@ -710,7 +739,7 @@ __global__ void __launch_bounds__(kRcWarps * 32) k_encode_rc(EncParams P, int la
             }
         }
         if (coded) {
-            code_corrections(e, P.corr + (size_t)item * kN3, ncorr);
+            code_corrections(e, P.pool + sy.w, ncorr);
             code_end(P, item, e.out, e.len, (uint64_t)e.ah << 32 | e.al, e.n, e.low);
         }
         __syncwarp();
@@ -802,8 +831,7 @@ coef:       // the coefficient at p - 1 (src/mc_codec.c:268-275)
         const uint32_t m = (uint32_t)(lv < 0 ? -lv : lv);
         w = ahead;
         pos = w & 0xFFFFu;
-        ahead = ent[min(idx, (uint32_t)kN3 - 1u)];
-        ++idx;
+        ahead = ent[idx++];   // up to two entries past the block's last (EncParams::pool)
         if (code_rung(e, g0, m > 1) && code_rung(e, g1, m > 2) && code_rung(e, g2, m > 3) && code_rung(e, g3, m > 4) &&
             code_rung(e, g4, m > 5) && code_rung(e, g5, m > 6) && code_rung(e, g6, m > 7) && code_rung(e, g7, m > 8) &&
             code_rung(e, g8, m > 9) && code_rung(e, g9, m > 10) && code_rung(e, g10, m > 11) &&
@@ -819,7 +847,7 @@ coef:       // the coefficient at p - 1 (src/mc_codec.c:268-275)
 __global__ void __launch_bounds__(32) k_encode_rc_one(EncParams P) {
     const int item = blockIdx.x;
     if (threadIdx.x) return;
-    const uint2 sy = P.sym[item];
+    const uint4 sy = P.sym[item];
     if (!(sy.x & 0x80000000u)) return;   // all air: not coded
     const uint32_t dc = sy.x & 0xFF, eob = (sy.x >> 8) & 0x1FFF, ncorr = sy.y;
     const EncItem it = P.items[item];
@@ -831,8 +859,8 @@ __global__ void __launch_bounds__(32) k_encode_rc_one(EncParams P) {
     e.range = 0xFFFFFFFFu;
     e.code = 0;
     code_header(e, [&qt](int j) { return (uint32_t)qt.ctx[j]; }, dc, eob, ncorr);
-    if (eob) code_scan(e, qt, P.entries + (size_t)item * kN3, eob);
-    code_corrections(e, P.corr + (size_t)item * kN3, ncorr);
+    if (eob) code_scan(e, qt, P.pool + sy.z, eob);
+    code_corrections(e, P.pool + sy.w, ncorr);
     code_end(P, item, e.out, e.len, e.code >> 32, e.n, (uint32_t)e.code);
 }
 
@@ -1222,6 +1250,23 @@ cudaError_t launch_encode_items(const EncChunks &c, EncItem *d_items, uint8_t *d
     return cudaGetLastError();
 }
 
+// One wave of CTAs: as many per SM as fit. CTAs walk the blocks with a fixed
+// stride, so CTAs beyond one wave would start their whole share late.
+static int encode_ctas(int n) {
+    static std::atomic<int> occ_by_dev[kMaxDevs];
+    const int occ = dev_once(occ_by_dev, [] {
+        int o = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_encode, 128, sizeof(EncSmem)) != cudaSuccess || o < 1) o = 1;
+        return o;
+    });
+    return std::min(n, dev_sms() * occ);
+}
+
+uint32_t encode_pool_max(int n) {
+    const uint32_t ctas = (uint32_t)encode_ctas(n);
+    return ctas * (((uint32_t)n + ctas - 1) / ctas) * (2u * kN3);
+}
+
 cudaError_t launch_encode(const EncParams &p, cudaStream_t s) {
     if (p.n <= 0) return cudaSuccess;
     const int smem = (int)sizeof(EncSmem);
@@ -1236,16 +1281,7 @@ cudaError_t launch_encode(const EncParams &p, cudaStream_t s) {
         return e == cudaSuccess ? 1 : -(int)e;
     });
     if (a < 0) return (cudaError_t)(-a);
-    const int sms = dev_sms();
-    // one wave of CTAs: as many per SM as fit. CTAs walk the blocks with a fixed
-    // stride, so CTAs beyond one wave would start their whole share late.
-    static std::atomic<int> occ_by_dev[kMaxDevs];
-    const int occ = dev_once(occ_by_dev, [smem] {
-        int o = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_encode, 128, smem) != cudaSuccess || o < 1) o = 1;
-        return o;
-    });
-    int blocks = p.n < sms * occ ? p.n : sms * occ;
+    const int blocks = encode_ctas(p.n);
     k_encode<<<blocks, 128, smem, s>>>(p);
     return cudaGetLastError();
 }

@@ -170,14 +170,22 @@ struct EncParams {
     const uint16_t *scan;
     uint32_t *len;       // per item: payload bytes (0 = all air, not coded)
     uint8_t *frac;       // per item: material nibble
-    uint32_t *status;    // [0]: payloads that overflowed kEncCap
-    // symbol scratch between the transform and the coder, per item: nonzero
-    // levels in scan order (kN3 u32: position | level << 16), corrections (kN3
-    // u32: pos | delta << 16), and (coded flag | eob << 8 | dc, ncorr)
-    uint32_t *entries;
-    uint32_t *corr;
-    uint2 *sym;
+    uint32_t *status;    // [0]: payloads that overflowed kEncCap, [1]: blocks that the pool had no room for
+    // symbols between the transform and the coder: per block its nonzero levels in
+    // scan order (position | level << 16) and its corrections (pos | delta << 16),
+    // one after the other in a pool of pool_words words, which k_encode's CTAs share
+    // evenly; and per item (coded flag | eob << 8 | dc, ncorr, where its levels
+    // start, where its corrections start). The coder reads up to two words past a
+    // block's levels: kEncPoolPad words must follow the pool.
+    uint32_t *pool;
+    uint32_t pool_words;
+    uint4 *sym;
 };
+constexpr uint32_t kEncPoolPad = 16;
+// Words for n blocks that hold 6144 symbols each: 4096 levels and half as many
+// corrections, where a block rarely has more than a few hundred of both.
+constexpr uint32_t encode_pool_words(uint32_t n) { return 6144u * n; }
+uint32_t encode_pool_max(int n);   // words that n blocks cannot exceed in launch_encode's shares
 cudaError_t upload_encode_tables(const float cmf[16][16], const uint16_t scan[kN3], cudaStream_t s);
 // Up to kEncChunks whole chunks of 256^3 voxels (c.vox[k], dense) as 4096 items
 // each, block by block, payload slots kEncCap bytes apart from d_pay on.

@@ -659,7 +659,7 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
         !L.b_fml.ensure(4 * nchunks) || !L.b_np.ensure(4 * nchunks) || !L.b_len.ensure(8 * nchunks) ||
         !L.b_off.ensure(8 * nchunks) || !L.b_q.ensure(4 * nchunks) || !L.h_misc.ensure(24 * (size_t)nchunks) ||
         !L.b_hash.ensure(8 * (size_t)nchunks) || !encode_streams(L) ||
-        !L.enc_ent.ensure(4 * (size_t)kN3 * n) || !L.enc_corr.ensure(4 * (size_t)kN3 * n) || !L.enc_sym.ensure(8 * n))
+        !L.enc_pool.ensure(4 * ((size_t)encode_pool_words((uint32_t)n) + kEncPoolPad)) || !L.enc_sym.ensure(sizeof(uint4) * n))
         return false;
     for (int c0 = 0; c0 < nchunks; c0 += kEncChunks) {
         EncChunks ec;
@@ -678,9 +678,7 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
     }
     float *hq = L.h_misc.as<float>();
     memcpy(hq, header_q, 4 * (size_t)nchunks);
-    if (!cuda_ok(cudaMemcpyAsync(L.b_q.p, hq, 4 * (size_t)nchunks, cudaMemcpyHostToDevice, L.stream), "H2D") ||
-        !cuda_ok(cudaMemsetAsync(L.status.p, 0, 16, L.stream), "memset"))
-        return false;
+    if (!cuda_ok(cudaMemcpyAsync(L.b_q.p, hq, 4 * (size_t)nchunks, cudaMemcpyHostToDevice, L.stream), "H2D")) return false;
     EncParams ep;
     ep.items = L.enc_items.as<EncItem>();
     ep.n = (int)n;
@@ -689,9 +687,7 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
     ep.len = L.enc_len.as<uint32_t>();
     ep.frac = L.enc_frac.as<uint8_t>();
     ep.status = L.status.as<uint32_t>();
-    ep.entries = L.enc_ent.as<uint32_t>();
-    ep.corr = L.enc_corr.as<uint32_t>();
-    ep.sym = L.enc_sym.as<uint2>();
+    ep.sym = L.enc_sym.as<uint4>();
     BlobParams bp;
     bp.nchunks = nchunks;
     bp.payload = L.enc_pay.as<uint8_t>();
@@ -709,25 +705,37 @@ bool encode_chunks(Lane &L, const uint8_t *const *d_vox, int nchunks, const floa
     bp.blobs = nullptr;
     bp.hash = L.b_hash.as<uint64_t>();
     // the fraction maps need the voxels only: beside the transform and the block coder
-    if (!cuda_ok(cudaEventRecord(L.ev_main, L.stream), "event record") ||
-        !cuda_ok(cudaStreamWaitEvent(L.side, L.ev_main, 0), "stream wait") ||
-        !cuda_ok(launch_fracmap(ep, bp, L.side), "fraction map launch") ||
-        !cuda_ok(cudaEventRecord(L.ev_side, L.side), "event record") ||
-        !cuda_ok(launch_encode(ep, L.stream), "encode launch") ||
-        !cuda_ok(launch_encode_rc(ep, L.stream), "range coder launch") ||
-        !cuda_ok(cudaStreamWaitEvent(L.stream, L.ev_side, 0), "stream wait") ||
-        !cuda_ok(launch_blob_layout(bp, L.stream), "blob layout launch")) {
+    bool ok = cuda_ok(cudaEventRecord(L.ev_main, L.stream), "event record") &&
+              cuda_ok(cudaStreamWaitEvent(L.side, L.ev_main, 0), "stream wait") &&
+              cuda_ok(launch_fracmap(ep, bp, L.side), "fraction map launch") &&
+              cuda_ok(cudaEventRecord(L.ev_side, L.side), "event record");
+    uint64_t *hl = reinterpret_cast<uint64_t *>(L.h_misc.as<uint8_t>() + 8 * (size_t)nchunks);
+    uint32_t status[2] = {0, 0};
+    while (ok) {
+        ep.pool = L.enc_pool.as<uint32_t>();
+        ep.pool_words = (uint32_t)std::min<size_t>(L.enc_pool.cap / 4 - kEncPoolPad, 0xFFFFFFFFu);
+        ok = cuda_ok(cudaMemsetAsync(L.status.p, 0, 16, L.stream), "memset") &&
+             cuda_ok(launch_encode(ep, L.stream), "encode launch") &&
+             cuda_ok(launch_encode_rc(ep, L.stream), "range coder launch") &&
+             cuda_ok(cudaStreamWaitEvent(L.stream, L.ev_side, 0), "stream wait") &&
+             cuda_ok(launch_blob_layout(bp, L.stream), "blob layout launch") &&
+             cuda_ok(cudaMemcpyAsync(hl, L.b_len.p, 8 * (size_t)nchunks, cudaMemcpyDeviceToHost, L.stream), "D2H") &&
+             cuda_ok(cudaMemcpyAsync(status, L.status.p, 8, cudaMemcpyDeviceToHost, L.stream), "D2H") &&
+             cuda_ok(cudaStreamSynchronize(L.stream), "encode sync");
+        if (!ok || !status[1]) break;
+        // more symbols than the pool holds (noise with a tight bound): once more with
+        // room for every block's most, which the lane then keeps
+        const size_t words = encode_pool_max((int)n);
+        if (ep.pool_words >= words) return set_error("encoder symbol pool overflow");
+        L.enc_pool.release();
+        ok = L.enc_pool.ensure(4 * (words + kEncPoolPad));
+    }
+    if (!ok) {
         cudaStreamSynchronize(L.side);   // nothing of this call outlives it
         cudaStreamSynchronize(L.stream);
         return false;
     }
-    uint64_t *hl = reinterpret_cast<uint64_t *>(L.h_misc.as<uint8_t>() + 8 * (size_t)nchunks);
-    uint32_t status = 0;
-    if (!cuda_ok(cudaMemcpyAsync(hl, L.b_len.p, 8 * (size_t)nchunks, cudaMemcpyDeviceToHost, L.stream), "D2H") ||
-        !cuda_ok(cudaMemcpyAsync(&status, L.status.p, 4, cudaMemcpyDeviceToHost, L.stream), "D2H") ||
-        !cuda_ok(cudaStreamSynchronize(L.stream), "encode sync"))
-        return false;
-    if (status) return set_error("block payload exceeded the encoder bound");
+    if (status[0]) return set_error("block payload exceeded the encoder bound");
     uint64_t total = 0;
     for (int c = 0; c < nchunks; ++c) {
         blob_len[c] = hl[c];

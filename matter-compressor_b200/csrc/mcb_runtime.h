@@ -103,7 +103,7 @@ struct Lane {
     DevBuf status, out;
     DecodeBatch batch;
     DevBuf enc_items, enc_len, enc_frac, enc_pay, src;
-    DevBuf enc_ent, enc_corr, enc_sym;   // encoder symbol scratch (entries, corrections, per-block info)
+    DevBuf enc_pool, enc_sym;                   // encoder symbols: levels and corrections, per-block info
     DevBuf b_scratch, b_lens16, b_bitmap, b_fmap, b_fml, b_np, b_len, b_off, b_q, b_hash, blobs;
     cudaStream_t side = nullptr;                // encoder: fraction maps beside the block coder, hashes beside the copy-out
     cudaEvent_t ev_side = nullptr, ev_main = nullptr;
