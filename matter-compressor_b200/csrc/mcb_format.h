@@ -98,4 +98,16 @@ MCB_HD inline uint32_t entry_cap(uint32_t len) {
 }
 constexpr uint32_t kEntryMax = 12288;
 
+// Length classes of the processing order: longer payloads in lower classes, absent
+// blocks in the last. Blocks of a class decode in about the same time: classes are 4
+// bytes wide to 2 KB, 16 to 6 KB and 256 beyond, 4 % of a length at most, up to the
+// 65535 bytes that a chunk's length table can give. (With everything from 4 KB on in
+// one class, 8 chunks of noise at q=0.25 took 32.2 ms per call.)
+constexpr int kLayoutClasses = 1024;
+MCB_HD inline int length_class(uint32_t len) {
+    const uint32_t l = len < 65535u ? len : 65535u;
+    const uint32_t k = l < 2048u ? l >> 2 : (l < 6144u ? 512u + ((l - 2048u) >> 4) : 768u + ((l - 6144u) >> 8));
+    return len ? kLayoutClasses - 2 - (int)k : kLayoutClasses - 1;
+}
+
 }  // namespace mcb

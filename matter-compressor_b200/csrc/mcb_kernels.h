@@ -87,7 +87,6 @@ cudaError_t launch_fused(const FusedParams &f, const LaunchCfg &cfg, cudaStream_
 // Arena offsets (base[i], entry_cap(len) entries each) and processing order
 // (longest payload first, absent blocks last) of n work items, on the device.
 // d_ws: kLayoutWords words.
-constexpr int kLayoutClasses = 1024;
 constexpr size_t kLayoutWords = 2 * kLayoutClasses + 2;   // counts, places taken, the arena's 64-bit total
 cudaError_t launch_layout(const DecItem *d_items, int n, uint64_t *d_base, uint32_t *d_order, uint32_t *d_ws,
                           cudaStream_t s);

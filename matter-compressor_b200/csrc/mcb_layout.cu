@@ -6,8 +6,8 @@
 // order only has to put similar lengths together (lanes of a warp then finish
 // about together, and the longest chains start first), so neither needs a full
 // scan or sort: a CTA reserves the entries of its 1024 items with one atomic, and
-// the order is a counting sort by length class of 4 bytes, whose ranks inside a
-// class fall as the CTAs arrive. On the host (a stable counting sort over 65536
+// the order is a counting sort by length class (see length_class), whose ranks inside
+// a class fall as the CTAs arrive. On the host (a stable counting sort over 65536
 // lengths, three more arrays built and uploaded) a batch of 46 K items took about
 // 0.3 ms of every call that builds its work list; here 10 us.
 #include <cuda_runtime.h>
@@ -21,13 +21,8 @@ namespace mcb {
 
 namespace {
 constexpr int kThreads = 1024;
-// class 0: payloads of 4092 bytes and more, ... class kClasses - 2: 1 to 3 bytes,
-// class kClasses - 1: absent
 constexpr int kClasses = kLayoutClasses;
 static_assert(kClasses == kThreads, "one thread per class in the scans");
-__device__ __forceinline__ int length_class(uint32_t len) {
-    return len ? kClasses - 2 - (int)min(len >> 2, (uint32_t)kClasses - 2) : kClasses - 1;
-}
 // Inclusive sum of v over the CTA's threads up to this one.
 __device__ __forceinline__ uint32_t cta_scan(uint32_t v, uint32_t *s_warp) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
