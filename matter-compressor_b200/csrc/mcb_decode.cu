@@ -328,15 +328,52 @@ __device__ __forceinline__ void decode_corrections(LaneState &L, const EntParams
     }
 }
 
+// Bits that a renormalisation shifts in (src/mc_codec.c:202): two bytes at
+// most, since the range is at least 2^24 before a bin and a split leaves at
+// least 15 * 2^12 of it (p <= 4081 once adapted).
+__device__ __forceinline__ uint32_t renorm_bits(uint32_t range) {
+    return range < (1u << 16) ? 16u : (range < kTop ? 8u : 0u);
+}
+
 // The rest of the coefficient at p - 1: for m > 12 the Exp-Golomb suffix of
 // m - 12 bits (the magnitude is 11 + (1 << nb | suffix), src/mc_codec.c:234-238,
 // 268-275), then sign and entry; false when the block ends (overflow pool
-// exhausted: corrupt streams only). The suffix of nb <= 16 bits is the
-// reference's batched read range >>= nb, q = min(code / range, 2^nb - 1),
-// code -= q * range: with the range's low nb bits cleared first, nb halvings
-// are that long division bit by bit, clamp included, and leave the same code
-// and range.
+// exhausted: corrupt streams only). A suffix of nb <= 16 bits, the batched read
+// range >>= nb, q = min(code / range, 2^nb - 1), code -= q * range (:216-226), and
+// the sign take at most 24 bits of the window, so both go straight through (see
+// renorm_bits): where many coefficients have a suffix, some lane of the warp is
+// here at every step (12 chunks at q=1 3.62 ms bit by bit with a renormalisation
+// loop each, 3.33 so; 10 chunks of noise at q=0.25 27.9 and 24.7).
 __device__ __forceinline__ bool finish_coef(LaneState &L, const EntParams &P, uint32_t m) {
+    const uint32_t nb = m > 12u ? m - 12u : 0u;
+    uint32_t neg;
+    if (nb <= 16u) {
+        uint32_t x = funnel_left(L.w2, L.w, L.used), code = L.code, r = L.range >> nb;
+        const uint32_t q = min(code / r, (1u << nb) - 1u);   // 0 without a suffix
+        code -= q * r;
+        m = nb ? 11u + ((1u << nb) | q) : m;
+        const uint32_t s1 = renorm_bits(r);
+        code = funnel_left(x, code, s1);
+        x <<= s1;
+        r = (r << s1) >> 1;
+        neg = code >= r ? 1u : 0u;
+        code = neg ? code - r : code;
+        const uint32_t s2 = r < kTop ? 8u : 0u;
+        L.code = funnel_left(x, code, s2);
+        L.range = r << s2;
+        L.used += s1 + s2;
+        if (L.used >= 32u) refill(L);
+    } else {
+        m = 11u + ((1u << (nb & 31u)) | bypass_long(L, nb));
+        neg = bypass_bits(L, 1);
+    }
+    return put_entry(L, P, (L.p - 1u) | ((neg ? 0u - m : m) << 16));
+}
+
+// The same with the suffix as nb halvings: with the range's low nb bits cleared
+// first they are that long division bit by bit, clamp included, and leave the same
+// code and range.
+__device__ __forceinline__ bool finish_coef_bits(LaneState &L, const EntParams &P, uint32_t m) {
     if (m > 12u) {
         const uint32_t nb = m - 12u;
         uint32_t acc = 1u << (nb & 31u);
@@ -360,7 +397,10 @@ __device__ __forceinline__ bool finish_coef(LaneState &L, const EntParams &P, ui
     return put_entry(L, P, (L.p - 1u) | ((neg ? 0u - m : m) << 16));
 }
 
-// The slow states of one lane, run while the rest of its warp waits.
+// The slow states of one lane, run while the rest of its warp waits. ALONE: of a
+// single-thread kernel, which gets here for S_END only; with finish_coef in its
+// place they still took 1 % longer (one chunk at q=0.5 2035 us, 2016 so).
+template <bool ALONE>
 __device__ __forceinline__ void slow_work(LaneState &L, const EntParams &P, uint32_t *ctx, const uint16_t *s_bend) {
     if (L.st == S_LAST) {
         uint32_t k = 0;
@@ -370,7 +410,8 @@ __device__ __forceinline__ void slow_work(LaneState &L, const EntParams &P, uint
                 if (++k >= 12u + (uint32_t)kEgCap) { L.bad = 1; L.st = S_DONE; return; }
             }
         }
-        if (finish_coef(L, P, k < 12u ? k + 1u : k)) L.st = S_END;
+        const uint32_t m = k < 12u ? k + 1u : k;
+        if (ALONE ? finish_coef_bits(L, P, m) : finish_coef(L, P, m)) L.st = S_END;
         return;
     }
     // S_END
@@ -400,13 +441,6 @@ __device__ __forceinline__ void fast_event(LaneState &L, const EntParams &P, con
     if (why & EV_CAP) { L.bad = 1; L.st = S_DONE; return; }
     if ((why & EV_OVF) && !put_entry(L, P, v)) return;   // pool exhausted, block ends
     if (L.p >= L.stop && L.k == 0) position_event(L, ctx, s_bend);
-}
-
-// Bits that a renormalisation shifts in (src/mc_codec.c:202): two bytes at
-// most, since the range is at least 2^24 before a bin and a split leaves at
-// least 15 * 2^12 of it (p <= 4081 once adapted).
-__device__ __forceinline__ uint32_t renorm_bits(uint32_t range) {
-    return range < (1u << 16) ? 16u : (range < kTop ? 8u : 0u);
 }
 
 // One step of every lane: up to a whole coefficient, by the same straight-line
@@ -545,7 +579,7 @@ __device__ __forceinline__ void run_lanes(LaneState &L, const EntParams &P, uint
     for (;;) {
         while (L.st >= S_LAST) {
             if (L.st != S_DONE) {
-                slow_work(L, P, ctx, s_bend);
+                slow_work<false>(L, P, ctx, s_bend);
                 continue;
             }
             if (L.item >= 0) {
@@ -755,7 +789,7 @@ position:
     if (L.st == S_LAST) goto coef;
 done:
     window_out(L);
-    while (L.st != S_DONE) slow_work(L, P, ctx, s_bend);
+    while (L.st != S_DONE) slow_work<true>(L, P, ctx, s_bend);
 }
 
 template <int WARPS>
