@@ -24,6 +24,13 @@ def sha(a):
     return hashlib.sha256(np.ascontiguousarray(a).tobytes()).hexdigest()
 
 
+def _arrays(name):
+    """The file's arrays, read at once: an open npz file reads each at its use,
+    which two threads of a test must not do at the same time."""
+    with np.load(os.path.join(GOLDEN, name)) as z:
+        return {k: z[k] for k in z.files}
+
+
 @pytest.fixture(scope="session")
 def oracle():
     from oracle import Oracle
@@ -51,22 +58,22 @@ def gpu():
 
 @pytest.fixture(scope="session")
 def golden_blocks():
-    return np.load(os.path.join(GOLDEN, "blocks.npz"))
+    return _arrays("blocks.npz")
 
 
 @pytest.fixture(scope="session")
 def golden_corrupt():
-    return np.load(os.path.join(GOLDEN, "corrupt.npz"))
+    return _arrays("corrupt.npz")
 
 
 @pytest.fixture(scope="session")
 def golden_meta():
-    return np.load(os.path.join(GOLDEN, "meta.npz"))
+    return _arrays("meta.npz")
 
 
 @pytest.fixture(scope="session")
 def golden_chunks():
-    return np.load(os.path.join(GOLDEN, "chunks.npz"))
+    return _arrays("chunks.npz")
 
 
 def ctx_q(q):
