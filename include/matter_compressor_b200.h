@@ -148,7 +148,7 @@ uint32_t mc_b200_last_bad_blocks(void);
  * blocks on single threads, the rest one per lane; 1: every block on a single
  * thread; 0: every block on a lane; -1 (the default): by the launch's
  * coded-block count (every block on single threads up to 19 K blocks, the
- * longest four per SM up to 200 K), and the longest 1/32 of a group in the
+ * longest four per SM up to 90 K), and the longest 1/32 of a group in the
  * host-blob pipeline, whose groups overlap. Decoded voxels
  * are the same in every case. Returns 0; -1 (with the last error set) for
  * share < -1 or without a usable device. No reference counterpart. */

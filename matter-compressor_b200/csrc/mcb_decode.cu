@@ -1895,11 +1895,14 @@ static cudaError_t launch_entropy_w(const EntParams &p, int ctas_per_sm, cudaStr
 // the launch's coded blocks. Below about 5 chunks' worth the stage's time is the
 // longest block's chain, which a single thread runs fastest (q=6: 2 chunks 352
 // us against 723 with lanes alone, 4 chunks 461 against 745; q=12: 244 against
-// 399). Up to about 60 chunks' worth the longest blocks, four for each SM (one
+// 399). Up to about 40 chunks' worth the longest blocks, four for each SM (one
 // for each of its schedulers), run on single threads beside the lanes (8 chunks
 // 637 us against 770 with lanes alone and 791 on single threads; 16: 745 / 850
-// / 1583; 32: 940 / 1055); a full 64 chunks gain nothing (1.55 ms).
-constexpr int kSoloAllMax = 19 * 1024, kSoloShareMax = 200 * 1024;
+// / 1583; 32: 940 / 1055). Beyond that the lanes are issue-bound and the single
+// threads' extra instructions cost more than their chains save: 40 chunks of noise
+// at q=0.25 68.8 ms with them, 63.4 without (q=0.1: 104 and 90), 48 chunks a third
+// air at q=1 12.1 and 11.9, at q=6 4.19 and 4.21.
+constexpr int kSoloAllMax = 19 * 1024, kSoloShareMax = 90 * 1024;
 static int auto_solo(int ncoded) {
     if (ncoded <= kSoloAllMax) return 1;
     return ncoded <= kSoloShareMax ? ncoded / (4 * num_sms()) : 0;

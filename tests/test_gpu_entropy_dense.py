@@ -43,3 +43,33 @@ def test_lanes_beside_single_threads(gpu, oracle, tmp_path):
             want = oracle.dec_block(a.block_blob(co, z, y, x), q).reshape(16, 16, 16)
             assert np.array_equal(got[0][16 * z:16 * z + 16, 16 * y:16 * y + 16, 16 * x:16 * x + 16], want), b
     assert took[0] < 0.65 * took[1], took
+
+
+def test_large_batches_on_lanes_alone(gpu, tmp_path):
+    """Beyond 90 K coded blocks the automatic split leaves the single threads out:
+    98304 blocks of noise in the time of lanes alone (1.10 of it with the longest
+    four of an SM on single threads)."""
+    import torch
+    q, n = 0.25, 24
+    g = torch.Generator(device="cuda").manual_seed(30)
+    v = (128 + torch.randn(256, 256, 256, device="cuda", generator=g) * 30).clamp(1, 255).to(torch.uint8)
+    out = torch.zeros(n, CHUNK, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    took = {}
+    with gpu.open(str(tmp_path / "l.mca"), 256, 256, 256, q) as a:
+        assert a.append_chunks(0, [(0, 0, 0)], [v.data_ptr()], q, on_device=True) == 0
+        co = a.chunk_offset(0, 0, 0, 0)
+        try:
+            for share in (0, -1):
+                assert gpu.L.mc_b200_set_entropy_solo(share) == 0
+                t = []
+                for _ in range(6):
+                    torch.cuda.synchronize()
+                    t0 = time.perf_counter()
+                    assert a.decode_chunks_dev([co] * n, out.data_ptr()) == 0
+                    torch.cuda.synchronize()
+                    t.append(time.perf_counter() - t0)
+                took[share] = min(t)
+        finally:
+            gpu.L.mc_b200_set_entropy_solo(-1)
+    assert took[-1] < 1.04 * took[0], took
