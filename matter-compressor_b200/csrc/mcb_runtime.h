@@ -115,6 +115,7 @@ struct Lane {
     HostBuf h_one;                              // single-block output, written by the kernel over the bus
     HostBuf h_bounce[3];                        // pieces between the device and pageable memory
     cudaEvent_t bounce_ev[3] = {};
+    uint32_t vox_up = 0;                        // chunks of several-chunk appends taken from host memory without them
     LaunchCfg cfg;
     BlobSlot pipe[kBlobSlots];
     ~Lane();
