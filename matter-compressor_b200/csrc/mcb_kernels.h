@@ -93,10 +93,9 @@ cudaError_t launch_layout(const DecItem *d_items, int n, uint64_t *d_base, uint3
 // The decode kernels' constant tables: the cosine basis and the band ends of
 // the scan order (scan position -> raster idx | band << 12).
 cudaError_t upload_decode_tables(const float cmf[16][16], const uint16_t scan[kN3], cudaStream_t s);
-// Loads the decode kernels' code now (first-call latency under lazy loading).
+// Load the decode kernels' code now (first-call latency under lazy loading).
 cudaError_t preload_decode_kernels();
-// Deblocking filter in place on `count` dense nz x ny x nx volumes vstride
-// bytes apart (three stream-ordered kernels: x, y, z faces).
+cudaError_t preload_layout_kernels();
 // LOD pyramid: 2x decimation of a dense dz x dy x dx volume into
 // ((dz+1)/2, (dy+1)/2, (dx+1)/2), and the gather of chunk (cz, cy, cx) of a
 // dense volume into a 256^3 buffer (zeros outside; *d_any |= 1 if non-zero).
@@ -108,6 +107,8 @@ cudaError_t launch_gather_chunk(const uint8_t *d_src, int nz, int ny, int nx, in
 // least min_frac over the gz x gy x gx block-fraction grid (nibbles 0..15).
 cudaError_t launch_sample_score(const uint8_t *d_grid, long gz, long gy, long gx, const long *d_cand, int n,
                                 long dz, long dy, long dx, float min_frac, uint8_t *d_accept, cudaStream_t s);
+// Deblocking filter in place on `count` dense nz x ny x nx volumes vstride bytes
+// apart: one kernel over tiles, or one per axis with faces, in stream order.
 cudaError_t launch_deblock(uint8_t *d_vol, int count, size_t vstride, int nz, int ny, int nx, int beta, int tc,
                            cudaStream_t s);
 // ---- serving ----

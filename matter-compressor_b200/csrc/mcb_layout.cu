@@ -90,4 +90,10 @@ cudaError_t launch_layout(const DecItem *d_items, int n, uint64_t *d_base, uint3
     return cudaGetLastError();
 }
 
+cudaError_t preload_layout_kernels() {
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, k_layout_count);
+    return e != cudaSuccess ? e : cudaFuncGetAttributes(&fa, k_layout_order);
+}
+
 }  // namespace mcb

@@ -91,8 +91,9 @@ static void runtime_init() {
     if (cudaMalloc(&R->d_scan, sizeof R->h_scan) != cudaSuccess ||
         cudaMalloc(&R->d_qtab, sizeof(QTab) * kMaxQSlots) != cudaSuccess ||
         cudaMemcpy(R->d_scan, R->h_scan, sizeof R->h_scan, cudaMemcpyHostToDevice) != cudaSuccess ||
-        upload_decode_tables(R->h_cos, R->h_scan, 0) != cudaSuccess || upload_encode_tables(R->h_cos, R->h_scan, 0) != cudaSuccess ||
-        preload_decode_kernels() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+        upload_decode_tables(R->h_cos, R->h_scan, 0) != cudaSuccess ||
+        upload_encode_tables(R->h_cos, R->h_scan, 0) != cudaSuccess || preload_decode_kernels() != cudaSuccess ||
+        preload_layout_kernels() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
         g_rt_err = std::string("device table upload failed: ") + cudaGetErrorString(cudaGetLastError());
         delete R;
         return;
