@@ -23,6 +23,18 @@ SOURCES = ["mcb_decode.cu", "mcb_encode.cu", "mcb_tables.cpp", "mcb_runtime.cpp"
            "mcb_archive.cpp", "mcb_api.cpp", "mcb_noalloc.cu", "mcb_gather.cu", "mcb_server.cpp", "mcb_deblock.cu", "mcb_lod.cu", "mcb_layout.cu", "mcb_sample.cu", "mcb_reader.cpp"]
 
 
+# The packed transforms keep their two roundings as this compiler orders them (see
+# csrc/mcb_f32x2.cuh); another one has to pass tests/test_transform_rounding.py first.
+NVCC_TESTED = "release 12.9"
+
+
+def _check_nvcc():
+    out = subprocess.run([NVCC, "--version"], check=True, capture_output=True, text=True).stdout
+    if NVCC_TESTED not in out:
+        print(f"build.py: nvcc is not {NVCC_TESTED}; run tests/test_transform_rounding.py on a GPU before using "
+              "this build", file=sys.stderr)
+
+
 def _stale(obj, deps):
     if not os.path.exists(obj):
         return True
@@ -35,6 +47,7 @@ def build(force=False, verbose=False):
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(HERE, "..", "include", "matter_compressor_b200.h"))
     objs = []
+    _check_nvcc()
     for src in SOURCES:
         path = os.path.join(CSRC, src)
         obj = os.path.join(BUILD, src + ".o")
