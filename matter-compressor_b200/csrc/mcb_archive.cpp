@@ -445,7 +445,7 @@ int mc_enc_block(mc_codec_ctx *C, const mc_u8 *vox, mc_buf *out, uint32_t *len_o
     int slot = qslot(C->quality);
     if (slot < 0) return 0;
     if (!cuda_ok(cudaEventSynchronize(L->done), "sync") || !L->src.ensure(kN3) || !L->enc_pay.ensure(kEncCap) ||
-        !L->enc_len.ensure(4) || !L->enc_frac.ensure(4) || !L->enc_items.ensure(sizeof(EncItem)) ||
+        !L->enc_len.ensure(4) || !L->enc_items.ensure(sizeof(EncItem)) ||
         !L->status.ensure(16) || !L->h_stage.ensure(kEncCap + 64) ||
         !L->enc_pool.ensure(4 * (2 * kN3 + kEncPoolPad)) || !L->enc_sym.ensure(sizeof(uint4)))
         return 0;
@@ -465,7 +465,7 @@ int mc_enc_block(mc_codec_ctx *C, const mc_u8 *vox, mc_buf *out, uint32_t *len_o
     ep.qtab = R->d_qtab;
     ep.scan = R->d_scan;
     ep.len = L->enc_len.as<uint32_t>();
-    ep.frac = L->enc_frac.as<uint8_t>();
+    ep.frac = nullptr;   // k_frac_count's, for chunks
     ep.status = L->status.as<uint32_t>();
     ep.pool = L->enc_pool.as<uint32_t>();
     ep.pool_words = 2 * kN3;

@@ -1011,26 +1011,11 @@ __device__ __forceinline__ void rec_init(float *sB) {
 // come from the shared table W.
 // On entry the coefficient box in sB, s_rec_ext and s_rec_l1 are zero; the
 // block leaves them zero again.
-// next: the item this CTA reconstructs after this one (-1: none). While this
-// block's transform runs, the start of the next block's entry list is
-// prefetched into L2, so that its loads do not wait on DRAM.
 template <bool CG>
 __device__ __forceinline__ void reconstruct_block(const RecParams &P, int item, float *sA, float *sB,
-                                                  uint8_t *stage, const float4 *W, int next = -1) {
+                                                  uint8_t *stage, const float4 *W) {
     const int tid = threadIdx.x;
     const int m = (tid & 3) * 2;
-    // the next block's entry window, fetched early (used after the dequantisation)
-    uint64_t nbase = 0;
-    uint32_t nlines = 0;
-    if (next >= 0 && tid < 32) {
-        // the entries it reads: coefficients and correction pairs, at most 512
-        nbase = __ldg(P.base + next);
-        const uint4 hv = __ldg(reinterpret_cast<const uint4 *>(P.hdr + next));
-        EntHdr hn;
-        memcpy(&hn, &hv, sizeof hn);
-        const uint32_t used = min((uint32_t)hn.nnz + 2u * hn.ncorr, entry_cap(__ldg(&P.items[next].len)));
-        nlines = (min(used, 512u) + 31) / 32;   // 128-byte lines
-    }
     const DecItem it = P.items[item];
     const EntHdr h = load_hdr<CG>(P.hdr + item);
     const uint64_t base = P.base[item];
@@ -1097,8 +1082,6 @@ __device__ __forceinline__ void reconstruct_block(const RecParams &P, int item, 
         E = s_rec_ext[0] + 1;
         const int Y = s_rec_ext[1] + 1, X = s_rec_ext[2] + 1;
         const bool fast = s_rec_l1 < kFastL1;
-        if ((uint32_t)tid < nlines)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(P.arena + nbase + 32ull * tid));
         // pass 1: lines along x for 4 adjacent cy at once, box[cz][k][cy..cy+3]
         // -> A[cz*Y + cy][x]. Group g of plane cz holds lines cy = 4g..4g+3;
         // lines at cy >= Y are zero and not stored. gi < 64, so

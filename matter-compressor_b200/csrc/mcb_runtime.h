@@ -111,7 +111,7 @@ struct Lane {
     DevBuf ver_items, ver_bad;                  // device verify: blob list, mismatch flags
     DevBuf smp_grid, smp_cand, smp_acc;         // box sampling: block-fraction grid, candidates, accept flags
     DevBuf solo;                                // single-block decode scratch (SoloScratch)
-    HostBuf h_items, h_base, h_stage, h_misc;
+    HostBuf h_stage, h_misc;
     HostBuf h_one;                              // single-block output, written by the kernel over the bus
     HostBuf h_bounce[3];                        // pieces between the device and pageable memory
     cudaEvent_t bounce_ev[3] = {};
