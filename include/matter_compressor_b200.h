@@ -148,10 +148,11 @@ uint32_t mc_b200_last_bad_blocks(void);
  * blocks on single threads, the rest one per lane; 1: every block on a single
  * thread; 0: every block on a lane; -1 (the default): by the launch's
  * coded-block count (every block on single threads up to 19 K blocks, the
- * longest four per SM up to 90 K), and the longest 1/32 of a group in the
- * host-blob pipeline, whose groups overlap. Decoded voxels
- * are the same in every case. Returns 0; -1 (with the last error set) for
- * share < -1 or without a usable device. No reference counterpart. */
+ * longest four per SM up to 90 K, none beyond); in the host-blob pipeline,
+ * whose groups overlap, the longest 1/32 of a group, none where pairs of blobs
+ * pass 10 MiB. Decoded voxels are the same in every case. Returns 0; -1 (with
+ * the last error set) for share < -1 or without a usable device. No reference
+ * counterpart. */
 int  mc_b200_set_entropy_solo(int share);
 
 /* Decode n whole chunk blobs held in HOST memory (blob i: blobs[i], blob_lens[i]

@@ -524,25 +524,20 @@ static bool blob_items(const uint8_t *b, uint64_t bl, const uint8_t *d_blob, Dec
 // Host blobs in, host voxels out, as a pipeline of kBlobSlots slots over
 // groups of kBlobGroup chunks: while one slot's voxels travel device->host,
 // the next slots' blobs travel host->device and decode. A slot is reused once
-// the event recorded after its previous group's copy-out has fired. A
-// group's decode takes about its longest block's serial chain, 1.5-1.7 ms at
-// q=6 whatever the group's size, so small groups with many in flight keep the
-// link busy soonest: 2-chunk groups over 8 slots reached 50.5 GB/s for 64
-// chunks where 8-chunk groups over 3 slots gave 49.1 (the plain device-to-host
-// copy on that box: 57.2 GB/s).
+// the event recorded after its previous group's copy-out has fired.
 int mc_b200_decode_chunk_blobs(const uint8_t *const *blobs, const uint64_t *lens, int n, mc_u8 *out,
                                size_t out_stride) {
     if (n < 0 || (n && (!blobs || !lens || !out))) return -1;
     Lane *L = lane();
     if (!L) return -1;
-    // 2 chunks per group when their blobs are small: the link binds, and a
-    // small first group starts it soonest (a q=6 pair is about 0.9 MB, q=3
-    // about 2.0 MB). 8 when two chunks' blobs pass 4 MiB (a q=1 pair is about
-    // 6.7 MB): the decode binds there and larger launches use the GPU better
-    // (q=1, 64 chunks: 34.2 GB/s end to end against 28.2 with 2-chunk groups;
-    // at q=3, 8-chunk groups gave 40.6 against 44.2)
+    // 2 chunks per group: a group's decode is about its longest block's chain
+    // whatever its size, so small groups with many in flight keep the link busy
+    // soonest (64 chunks at q=6 20.1 ms, 20.9 in groups of 8; at q=1, 6.4 MiB a pair,
+    // 24.2 and 28.0). 8 when a pair of blobs passes 10 MiB: the decode binds there and
+    // larger launches use the GPU better (64 chunks of material at q=0.5, 13.5 MiB a
+    // pair, 39.7 ms against 49.1; q=0.25, 18.6 MiB, 53.6 against 88.8)
     constexpr int kBlobGroupMax = 8, kBlobGroupSmall = 2;
-    constexpr uint64_t kBigPairBytes = 4ull << 20;
+    constexpr uint64_t kBigPairBytes = 10ull << 20;
     bool ok = true;
     for (int k = 0; k < kBlobSlots; ++k) ok = ok && blob_slot_ready(L->pipe[k]);
     uint32_t bad = 0;
@@ -584,9 +579,11 @@ int mc_b200_decode_chunk_blobs(const uint8_t *const *blobs, const uint64_t *lens
         // instructions per bin count, but for the few longest blocks, whose chains
         // hold the group's copy-out back (64 chunks at q=6 20.23 ms with lanes
         // alone, 20.13 so, 20.56 with every block on a single thread; 16 chunks at
-        // q=1 10.17, 9.93, 15.85; 3 chunks at q=6 1.79, 1.65, 1.61)
+        // q=1 8.7, 8.6). Not where the decode binds: 64 chunks of material at q=0.25
+        // 53.6 ms with lanes alone, 62.7 with the longest 1/32 on single threads (one
+        // group of 4 at q=0.5 7.5 and 6.6).
         LaunchCfg cfg = L->cfg;
-        if (cfg.ent_solo < 0) cfg.ent_solo = 32;
+        if (cfg.ent_solo < 0) cfg.ent_solo = pair > kBigPairBytes && n > g ? 0 : 32;
         ok = ok && decode_prepare_staged(B, (int)ni, S.stream) && decode_enqueue(B, cfg, S.stream) &&
              cuda_ok(cudaMemcpyAsync(B.h_status.p, B.status.p, 4, cudaMemcpyDeviceToHost, S.stream), "D2H status");
         if (!ok) break;

@@ -73,3 +73,37 @@ def test_large_batches_on_lanes_alone(gpu, tmp_path):
         finally:
             gpu.L.mc_b200_set_entropy_solo(-1)
     assert took[-1] < 1.04 * took[0], took
+
+
+def test_pipeline_of_dense_blobs(gpu, tmp_path):
+    """Host blobs whose decode binds (26 MiB a pair) in the time of lanes alone: 32
+    chunks took 1.2 times as long with the longest 1/32 of a group on single threads."""
+    import torch
+    from mcb200 import Reader, decode_chunk_blobs
+    q, n = 0.25, 32
+    g = torch.Generator(device="cuda").manual_seed(30)
+    v = (128 + torch.randn(256, 256, 256, device="cuda", generator=g) * 20).clamp(1, 255).to(torch.uint8)
+    torch.cuda.synchronize()
+    path = str(tmp_path / "b.mca")
+    with gpu.open(path, 256, 256, 256, q) as a:
+        assert a.append_chunks(0, [(0, 0, 0)], [v.data_ptr()], q, on_device=True) == 0
+        co = a.chunk_offset(0, 0, 0, 0)
+        want = a.decode_chunk(co).copy()
+    with Reader(gpu, data=np.fromfile(path, np.uint8)) as r:
+        blob = torch.from_numpy(np.frombuffer(r.blob(co), np.uint8).copy()).pin_memory().numpy()
+    assert blob.size > 10 << 20
+    out = torch.zeros(n * CHUNK, dtype=torch.uint8).pin_memory().numpy()
+    took = {}
+    try:
+        for share in (0, -1):
+            assert gpu.L.mc_b200_set_entropy_solo(share) == 0
+            t = []
+            for _ in range(6):
+                t0 = time.perf_counter()
+                decode_chunk_blobs(gpu, [blob] * n, out=out)
+                t.append(time.perf_counter() - t0)
+            took[share] = min(t)
+            assert all(np.array_equal(out[k * CHUNK:(k + 1) * CHUNK], want) for k in (0, 7, 8, n - 1))
+    finally:
+        gpu.L.mc_b200_set_entropy_solo(-1)
+    assert took[-1] < 1.05 * took[0], took
