@@ -460,13 +460,13 @@ __device__ __forceinline__ void fast_event(LaneState &L, const EntParams &P, con
 // itself. The context values come from shared memory a step ahead (ps, pm):
 // loaded as soon as the next position's density class and the next rung are
 // known, after the store of the context just used.
-// One step reads at most 40 bits (see renorm_bits), the window always holds
-// at least 40, and the 32 extracted here serve all but a sign after more than
-// 24 bits, which is left to fast_event. Returns the events of the lane; v is
-// its entry (for EV_COEF, the argument of finish_coef in the high half).
+// The bins of a step could take 40 bits (see renorm_bits), and the window always
+// holds as many; the 32 extracted here serve all but a sign after more than 24 bits,
+// which is left to fast_event. Returns the events of the lane; v is its entry (for
+// EV_COEF, the argument of finish_coef in the high half).
 // What bounds it: integer issue, most of it on the ALU pipe at half rate. Runs
-// of length 1 or 4: allowing 1 to 4 takes 5 % fewer steps (of a q=6 sample: 424
-// against 445, 1028 without runs) of a tenth more instructions. A step of one
+// of length 1 or 4: allowing 1 to 4 takes 6 % fewer steps (a q=6 block of the bench
+// volumes 701 against 743, 1643 without runs) of a tenth more instructions. A step of one
 // bin per lane took 2041 steps a block at q=6 and 9870 at q=1; 64 chunks at
 // q=6: 2.68 ms with it, 1.54 ms with this one.
 __device__ __forceinline__ uint32_t fast_step(LaneState &L, const EntParams &P, uint32_t *ctx, uint32_t &v) {
@@ -1354,8 +1354,9 @@ __device__ __forceinline__ void pass3(const float4 *in, int E, int half, int dc,
 // outputs at a time and takes its weights from constant memory by a warp-uniform
 // index; all sums are packed adds (see lines4p).
 // What bounds it: latency, at 18 warps an SM and 0.43 instructions a cycle and
-// scheduler (3130 a block at q=6, 3960 before). 64 chunks at q=6 1.61 ms, at q=12
-// 1.16; with reconstruct_block on 4-warp CTAs 1.87 and 1.51. Tried and dropped:
+// scheduler (3130 a block at q=6, 3960 before). 64 chunks at q=6 1.55 ms, at q=12
+// 1.15 (1.61 and 1.16 without the pairs of launch_reconstruct); with reconstruct_block on
+// 4-warp CTAs 1.87 and 1.51. Tried and dropped:
 // one warp per block without barriers (10 warps an SM, 1.87), pairs of blocks
 // with 32-byte row stores (16 registers held over a block, spills: 1.70).
 __global__ void __launch_bounds__(64, 9) k_reconstruct(RecParams P) {
@@ -1573,7 +1574,7 @@ __global__ void __launch_bounds__(64, 9) k_reconstruct(RecParams P) {
 // ---------------------------------------------------------------- fused decode
 // One persistent kernel for both stages. Every CTA first runs entropy lanes
 // (the k_entropy loop) until the shared block queue is drained. Blocks are
-// reconstructed in the pairs k_reconstruct uses (items 2j, 2j+1, x-neighbours
+// reconstructed in pairs (items 2j, 2j+1, x-neighbours
 // inside a chunk): the block that completes a pair -- an absent block at
 // kernel start, a coded one when its lane finishes -- appends the pair to a
 // completion list. A CTA whose lanes are all idle reconstructs pairs in list

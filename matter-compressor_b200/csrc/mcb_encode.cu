@@ -901,7 +901,8 @@ __global__ void __launch_bounds__(256) k_frac_count(EncParams P) {
 // (four 1 bins); such a nibble is coded straight through, the four splits
 // computed one from the other, when the last range shows that none of them
 // renormalises. One chunk or many: 0.95 ms as the tail of the sizing pass with
-// contexts in local memory, 0.75 ms here and hidden.
+// contexts in local memory, 0.75 ms here, hidden where the transform and the block
+// coder take longer (not for the small levels of a pyramid).
 __device__ __forceinline__ void frac_bit(Enc &e, uint32_t &p0, uint32_t bit) {
     const uint32_t r0 = (e.range >> 12) * p0;
     if (!bit) { e.range = r0; p0 = after0(p0); }

@@ -14,7 +14,8 @@ namespace mcb {
 // block (madd2 in mcb_decode.cu) the multiply is packed and the adds are scalar
 // __fadd_rn, a combination that keeps both roundings; packed adds take sums, and
 // products that arrive through a loop's back edge (lines4p and pass3 there,
-// dct_lines and idct_lines in mcb_encode.cu).
+// dct_lines and idct_lines in mcb_encode.cu). tests/test_transform_rounding.py holds
+// inputs that a contraction anywhere in them changes.
 __device__ __forceinline__ float2 add2(float2 a, float2 b) {
     float2 d;
     asm("{.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"

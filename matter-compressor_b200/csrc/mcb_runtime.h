@@ -126,9 +126,9 @@ bool decode_prepare(DecodeBatch &B, const DecItem *h_items, int n, cudaStream_t 
 // decode_prepare without any host synchronisation: the n items are already in
 // B.h_items (pinned) and are uploaded asynchronously on s, where order and
 // offsets are then made by the device (mcb_layout.cu); a batch beyond one
-// arena is laid out in sub-batches in B's pinned staging instead. No split-off
-// long blocks (DecodeBatch::split) either way: that is a plan's layout. The
-// caller guarantees that the batch's previous use has completed.
+// arena is laid out in sub-batches in B's pinned staging instead. Launches without
+// a plan use no split-off long blocks (DecodeBatch::split). The caller guarantees
+// that the batch's previous use has completed.
 bool decode_prepare_staged(DecodeBatch &B, int n, cudaStream_t s);
 // Creates the stream and event of a pipeline slot on first use.
 bool blob_slot_ready(BlobSlot &S);
